@@ -38,15 +38,15 @@ EXACT_MATH = {"conv_norm", "depth_average", "diff_attention", "diff_prefill", "l
               "window_attention", "window_prefill"}
 # sources one served architecture needs: ``ensure_kernels`` builds only these when the full library is not there
 KERNEL_SETS = {
-    "nafitar": ("comm", "elementwise", "gemm_skinny", "gemm_tcgen05", "gemm_wide", "matrix_memory", "matrix_memory_chunk",
-                "sample_filtered", "sandwich_norm", "vocab", "window_attention", "window_prefill"),
-    "kedesun": ("attention_fwd", "comm", "depth_average", "elementwise", "gemm_skinny", "gemm_tcgen05", "gemm_wide",
+    "nafitar": ("comm", "elementwise", "gemm_skinny", "gemm_stream", "gemm_tcgen05", "gemm_wide", "matrix_memory",
+                "matrix_memory_chunk", "sample_filtered", "sandwich_norm", "vocab", "window_attention", "window_prefill"),
+    "kedesun": ("attention_fwd", "comm", "depth_average", "elementwise", "gemm_skinny", "gemm_stream", "gemm_tcgen05", "gemm_wide",
                 "latent_attention", "matrix_memory", "matrix_memory_chunk", "mla_decode", "moe_serve", "router",
                 "sample_filtered", "sandwich_norm", "vocab", "window_attention"),
-    "lobutar": ("attention_fwd", "comm", "diff_attention", "diff_prefill", "elementwise", "gemm_skinny", "gemm_tcgen05",
+    "lobutar": ("attention_fwd", "comm", "diff_attention", "diff_prefill", "elementwise", "gemm_skinny", "gemm_stream", "gemm_tcgen05",
                 "gemm_wide", "latent_attention", "mla_decode", "moe_serve", "router", "sample_filtered", "sandwich_norm",
                 "stream_mix", "vocab", "window_attention"),
-    "rezulorn": ("comm", "conv_norm", "elementwise", "gemm_skinny", "gemm_tcgen05", "gemm_wide", "matrix_memory",
+    "rezulorn": ("comm", "conv_norm", "elementwise", "gemm_skinny", "gemm_stream", "gemm_tcgen05", "gemm_wide", "matrix_memory",
                  "matrix_memory_chunk", "moe_serve", "sample_filtered", "scored_attention", "scored_prefill", "vocab",
                  "window_attention"),
 }

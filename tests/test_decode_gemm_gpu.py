@@ -1,0 +1,39 @@
+"""The weight-streaming decode GEMM against fp32, where its three ways to cut the work meet their edges."""
+import pytest
+import torch
+
+from gcore_b200.ops import _lib
+from gcore_b200.ops import gemm as G
+
+pytestmark = pytest.mark.gpu
+
+
+# (N, K): one piece per CTA with equal and unequal pieces, ragged tiles and k-blocks, runs that divide tiles, runs of whole
+# tiles, one tile more than SMs
+SHAPES = [(3584, 3584), (4608, 1600), (700, 9000), (7168, 1152), (24576, 512), (32768, 520), (19072, 712), (300, 20000)]
+
+
+@pytest.mark.parametrize("N,K", SHAPES)
+@pytest.mark.parametrize("T", [1, 16, 17, 63, 128])
+def test_stream_gemm(N, K, T):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    g = torch.Generator(device="cuda").manual_seed(N + K + T)
+    x = torch.randn(T, K, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    b = torch.randn(N, generator=g, device="cuda")
+    ref = x.double() @ w.double().t()
+    before = G.LAUNCHES["gemm"]
+    y = G.linear_forward(x, w, out_dtype=torch.float32)
+    assert N * K >= 5 << 20 and G.LAUNCHES["gemm"] == before + 1
+    # fp32 sums of K products of exact bf16 values: sqrt(K) roundings of 2^-24 relative to the sum of magnitudes
+    bound = 4 * K ** 0.5 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    assert ((y.double() - ref).abs() <= bound + 1e-12).all()
+    yb = G.linear_forward(x, w, b.bfloat16())
+    refb = ref + b.bfloat16().double()
+    assert ((yb.double() - refb).abs() <= refb.abs() * 2.0 ** -8 + bound + 1e-12).all()
+    out = torch.full((T, N + 24), 7.0, device="cuda", dtype=torch.float32)[:, 8:N + 8]     # strided result
+    G.linear_forward(x, w, b, out=out)
+    assert torch.equal(out, G.linear_forward(x, w, b, out_dtype=torch.float32))
+    assert bool((out._base[:, :8] == 7).all()) and bool((out._base[:, N + 8:] == 7).all())
+    _lib.check_device_errors()
