@@ -4,8 +4,9 @@
 //   * swap-AB: the 128-row tcgen05 tile runs over output features, the token count is the MMA N (16 .. 128).
 //   * Few feature tiles (up to half the SMs): every tile is cut along K into as many equal pieces as there are SMs per
 //     tile, one piece per CTA.  The pieces of a tile lie in fp32 in a scratch buffer (they stay in L2); each of its CTAs
-//     waits for the others' and adds its share of the tile.  (All CTAs of the grid are resident, one per SM at most,
-//     which the wait relies on.)
+//     waits for the others' and adds its share of the tile.  The CTAs of a grid usually run at the same time, one per SM
+//     at most, and wait a microsecond or two; one that waits long (kernels of other streams hold the SMs) leaves its
+//     share to the CTA that brings the last piece, so that nothing depends on all of them being resident.
 //   * More tiles: the sequence of (tile, 64-deep k-block) units, tile after tile, is cut into one contiguous run per SM, so
 //     that 192 or 296 tiles stream as evenly as a multiple of 148; the CTA that brings a divided tile's last piece adds
 //     them up.  (Waiting for the others would cost: a run's first piece belongs to a tile that its neighbour ends with.)
@@ -18,6 +19,9 @@
 // columns each).  Two accumulators: a piece is drained while the next one is contracted.
 #include "ptx.cuh"
 #include "host_utils.h"
+#include <map>
+#include <mutex>
+#include <utility>
 
 namespace gkst {
 using namespace gk;
@@ -39,7 +43,7 @@ struct StParams {
   const void* bias;
   int bias_fp32;
   float* ws;       // [CTA][first, last piece][Tp tokens][128 features]
-  int* counters;   // [tiles][pieces there, CTAs done with them], zero between launches
+  unsigned long long* counters;   // [tiles]: pieces there | CTAs done << 8 | shares left over << 16, zero between launches
   int* err;
 };
 
@@ -82,11 +86,13 @@ __device__ __forceinline__ void store_cols(const StParams& p, const float (&v)[C
   }
 }
 
-__device__ __forceinline__ int load_acquire(const int* a) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
+__device__ __forceinline__ unsigned long long load_acquire(const unsigned long long* a) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(a) : "memory");
   return v;
 }
+constexpr int MAX_PIECES = 48;             // shares of a tile the counter word has a bit for
+constexpr long long SHARE_WAIT = 100000;   // cycles, about 50 us
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
 // Adds up items [i0, i1) of a divided tile, an item being four features of one token.
@@ -122,43 +128,52 @@ __device__ __forceinline__ void sum_pieces(const StParams& p, int tile, int lo, 
 
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
 
-// What follows when this CTA's piece of a divided tile lies in the scratch.  Returns false when a wait ran out.
-__device__ __forceinline__ bool finish_piece(const StParams& p, int tile, int ctas, int* s_flag) {
+// What follows when this CTA's piece of a divided tile lies in the scratch.
+__device__ __forceinline__ void finish_piece(const StParams& p, int tile, int ctas, unsigned long long* s_word) {
   int lo, hi;
   tile_owners(p, tile, ctas, lo, hi);
   const int pieces = hi - lo + 1, items = 32 * p.T;
-  int* there = &p.counters[2 * tile];
-  bool ok = true;
+  unsigned long long* word = &p.counters[tile];
   __threadfence();
   epi_sync();
   if (p.ks) {
+    const int mine = static_cast<int>(blockIdx.x) - lo;
     if (threadIdx.x == 64) {
-      atomicAdd(there, 1);
-      const long long t0 = clock64();
-      bool all = true;
-      while (all && load_acquire(there) < pieces) {
-        if (clock64() - t0 > WAIT_BUDGET_CYCLES) { atomicCAS(p.err, 0, ERR_WAIT_MISC); all = false; }
-        if (*reinterpret_cast<volatile int*>(p.err) != 0) all = false;
+      unsigned long long shares = 1ull << mine;     // what this CTA adds up
+      const unsigned long long old = atomicAdd(word, 1ull);
+      if (static_cast<int>(old & 0xff) == pieces - 1) {
+        shares |= old >> 16;
+      } else {
+        const long long t0 = clock64();
+        while (static_cast<int>(load_acquire(word) & 0xff) < pieces) {
+          if (clock64() - t0 < SHARE_WAIT) continue;
+          // the CTA that brings the last piece sees the bit, unless it came first: then all pieces are there
+          if (static_cast<int>(atomicOr(word, shares << 16) & 0xff) < pieces) shares = 0;
+          break;
+        }
       }
-      *s_flag = all ? 1 : 0;
+      __threadfence();
+      *s_word = shares;
     }
     epi_sync();
-    ok = *s_flag != 0;
-    const int mine = static_cast<int>(blockIdx.x) - lo;
-    if (ok) sum_pieces(p, tile, lo, hi, items * mine / pieces, items * (mine + 1) / pieces);
-    // the last CTA to have seen all pieces leaves the counters at zero for the next launch
-    if (threadIdx.x == 64 && ok && atomicAdd(there + 1, 1) == pieces - 1) { there[0] = 0; there[1] = 0; }
+    for (unsigned long long shares = *s_word; shares; shares &= shares - 1) {
+      const int k = __ffsll(shares) - 1;
+      sum_pieces(p, tile, lo, hi, items * k / pieces, items * (k + 1) / pieces);
+    }
+    // the last CTA to be done leaves the word at zero for the next launch
+    if (threadIdx.x == 64 && static_cast<int>((atomicAdd(word, 256ull) >> 8) & 0xff) == pieces - 1) *word = 0;
   } else {
-    if (threadIdx.x == 64) *s_flag = atomicAdd(there, 1) == pieces - 1 ? 1 : 0;
-    epi_sync();
-    if (*s_flag) {
+    if (threadIdx.x == 64) {
+      *s_word = static_cast<int>(atomicAdd(word, 1ull)) == pieces - 1;
       __threadfence();
+    }
+    epi_sync();
+    if (*s_word) {
       sum_pieces(p, tile, lo, hi, 0, items);
-      if (threadIdx.x == 64) there[0] = 0;
+      if (threadIdx.x == 64) *word = 0;
     }
     epi_sync();   // the flag may be written again
   }
-  return ok;
 }
 
 __global__ void __launch_bounds__(THREADS, 2)
@@ -171,7 +186,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   uint64_t* tfull = empty + MAX_STAGES;   // 2
   uint64_t* tempty = tfull + 2;           // 2
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty + 2);
-  int* s_flag = reinterpret_cast<int*>(tmem_holder + 1);
+  unsigned long long* s_word = reinterpret_cast<unsigned long long*>(tmem_holder + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ctas = gridDim.x;
@@ -286,7 +301,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
       tc_fence_before();
       mbar_arrive(&tempty[acc]);
-      if (!whole) ok = finish_piece(p, tile, ctas, s_flag);
+      if (!whole) finish_piece(p, tile, ctas, s_word);
       u = next;
     }
   }
@@ -302,25 +317,60 @@ static int padded_tokens(int T) { return (T + 15) / 16 * 16; }
 
 using namespace gkst;
 
-// Identity of the capture the stream is in, 0 outside of one.
-GK_EXPORT long long gk_capture_id(void* stream) {
+// Counters of the divided tiles.  A launch leaves them at zero; launches that may run at the same time must not share them:
+// every stream has a slot of its own, and so has every stream of a capture (a graph may be replayed anywhere).  Captures
+// take the upper half of the slots in turn, streams the lower half.  The buffer is the caller's (one per device, zeroed).
+namespace {
+struct CounterPool {
+  int* base = nullptr;
+  int slots = 0, ints = 0, next[2] = {0, 0};
+  std::map<std::pair<unsigned long long, cudaStream_t>, int> taken;   // (capture, 0 outside of one; stream) -> slot
+};
+std::mutex pools_mutex;
+std::map<int, CounterPool> pools;   // by device
+
+int* counters_of(cudaStream_t st, int need) {
+  int dev = 0;
   cudaStreamCaptureStatus status;
   unsigned long long id = 0;
-  if (cudaStreamGetCaptureInfo(reinterpret_cast<cudaStream_t>(stream), &status, &id) != cudaSuccess) {
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) {
     cudaGetLastError();
-    return 0;
+    return nullptr;
   }
-  return status == cudaStreamCaptureStatusActive ? static_cast<long long>(id) : 0;
+  const int half = status == cudaStreamCaptureStatusActive ? 1 : 0;
+  std::lock_guard<std::mutex> lock(pools_mutex);
+  CounterPool& pool = pools[dev];
+  if (!pool.base || pool.ints < need) return nullptr;
+  if (pool.taken.size() >= 4u * pool.slots) pool.taken.clear();
+  auto [it, fresh] = pool.taken.try_emplace({half ? id : 0ull, st}, 0);
+  if (fresh) {
+    it->second = pool.next[half] + half * (pool.slots / 2);
+    pool.next[half] = (pool.next[half] + 1) % (pool.slots / 2);
+  }
+  return pool.base + static_cast<long long>(it->second) * pool.ints;
+}
+}  // namespace
+
+// The current device's counters: `slots` (even) times `ints` (even) zeroed ints, 8-byte aligned.
+GK_EXPORT int gk_gemm_stream_pool(int* base, int slots, int ints) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || slots < 2 || slots % 2 || ints % 2 || (reinterpret_cast<uintptr_t>(base) & 7)) return -1;
+  std::lock_guard<std::mutex> lock(pools_mutex);
+  CounterPool& pool = pools[dev];
+  pool.base = base; pool.slots = slots; pool.ints = ints;
+  pool.next[0] = pool.next[1] = 0;
+  pool.taken.clear();
+  return 0;
 }
 
 // Floats of scratch for the pieces of divided tiles.
 GK_EXPORT long long gk_gemm_stream_scratch(int T) { return 2ll * sm_count() * padded_tokens(T) * BM; }
 
 // W [N, K] and X [T, K] bf16 row-major (K contiguous, leading dimensions multiples of 8, 16-byte aligned), 1 <= T <= 128;
-// counters: two per 128 features, zero before the launch, left zero by it, not shared with launches that may run meanwhile.
+// the device's pool of counters has to hold two per 128 features in a slot (-9 without).
 GK_EXPORT int gk_gemm_stream(const void* W, long long ldw, const void* X, long long ldx, void* Y, long long ldy,
                              int out_fp32, const void* bias, int bias_fp32, int T, int N, int K, float* ws,
-                             long long ws_floats, int* counters, long long n_counters, int* err, void* stream) {
+                             long long ws_floats, int* err, void* stream) {
   if (T < 1 || T > 128 || N < 1 || K < 1) return -1;
   if ((ldw & 7) || (ldx & 7) || (reinterpret_cast<uintptr_t>(W) & 15) || (reinterpret_cast<uintptr_t>(X) & 15)) return -3;
   StParams p;
@@ -329,12 +379,14 @@ GK_EXPORT int gk_gemm_stream(const void* W, long long ldw, const void* X, long l
   p.kbs = (K + BK - 1) / BK;
   if (static_cast<long long>(tiles) * p.kbs > 0x3fffffff) return -2;
   p.units = tiles * p.kbs;
-  if (ws_floats < gk_gemm_stream_scratch(T) || n_counters < 2ll * tiles) return -8;
+  if (ws_floats < gk_gemm_stream_scratch(T)) return -8;
+  int* counters = counters_of(reinterpret_cast<cudaStream_t>(stream), 2 * tiles);
+  if (!counters) return -9;
   CUtensorMap tmW, tmX;
   if (make_tmap_2d(&tmW, W, 2, N, K, ldw, BM, BK, true)) return -4;
   if (make_tmap_2d(&tmX, X, 2, T, K, ldx, p.Tp, BK, true)) return -5;
   p.Y = Y; p.ldy = ldy; p.out_fp32 = out_fp32; p.bias = bias; p.bias_fp32 = bias_fp32;
-  p.ws = ws; p.counters = counters; p.err = err;
+  p.ws = ws; p.counters = reinterpret_cast<unsigned long long*>(counters); p.err = err;
   const int sms = sm_count(), stage_bytes = A_BYTES + p.Tp * 128;
   const double weight_us = 2e-6 * N * K / 6.5;   // time the weight takes from HBM
   // Ring: below half of an SM the next GEMM's CTA fits beside this one and has its first loads under way early; that pays
@@ -353,7 +405,8 @@ GK_EXPORT int gk_gemm_stream(const void* W, long long ldw, const void* X, long l
     const int most = p.kbs / 3 > 1 ? p.kbs / 3 : 1;   // at least three k-blocks per piece
     const bool full = tiles * ks * 5 >= sms * 4;
     if (ks > most) ks = most;
-    if (full || ks == most || T > 64) { p.ks = ks; grid = tiles * ks; }
+    if (ks > MAX_PIECES) ks = MAX_PIECES;
+    if (full || ks == most || ks == MAX_PIECES || T > 64) { p.ks = ks; grid = tiles * ks; }
   }
   // Adding up divided tiles costs about 1.5 us and 0.1 us per token; whole tiles leave SMs idle in the last round
   // (32768 x 1024, 64 tokens: 22.6 in runs, 18.2 in whole tiles; 28672 x 4096, 4 tokens: 42 against 52).

@@ -274,31 +274,22 @@ def _skinny_plan(T: int, tiles: int, kb: int, K: int):
 
 STREAM = {"enabled": os.environ.get("GCORE_STREAM_GEMM", "1") != "0"}
 COUNTER_SLOTS, SLOT_INTS = 256, 8192
-_COUNTERS: dict = {}   # device index -> (zeroed counters of all slots, {stream or capture: slot})
+_COUNTERS: dict = {}        # device index -> zeroed counters of all slots
+_STREAM_SCRATCH: dict = {}  # tokens -> floats of scratch
 
 
-def _stream_counters(device):
-    """Zeroed counters of the streaming decode GEMM (every launch leaves them zero) for the current stream, or, while it is
-    being captured, for this capture: launches that may run at the same time must not share them.  None when there are none
-    yet and none can be made (inside a capture)."""
-    stream = torch.cuda.current_stream(device).cuda_stream
-    capture = _lib.kernels().gk_capture_id(ctypes.c_void_p(stream))
+def _stream_ready(device, N: int) -> bool:
+    """Gives the library its zeroed counters on a device's first use.  False inside a capture (they cannot be made there)
+    and for more tiles than a slot counts."""
     if device.index not in _COUNTERS:
-        if capture:
-            return None
-        _COUNTERS[device.index] = (torch.zeros(COUNTER_SLOTS, SLOT_INTS, dtype=torch.int32, device=device), {})
+        if torch.cuda.is_current_stream_capturing():
+            return False
+        counters = torch.zeros(COUNTER_SLOTS, SLOT_INTS, dtype=torch.int32, device=device)
         torch.cuda.current_stream(device).synchronize()   # once: other streams use it without waiting for this one
-    counters, slots = _COUNTERS[device.index]
-    key = (capture, 0) if capture else (0, stream)
-    slot = slots.get(key)
-    if slot is None:
-        if len(slots) >= 4 * COUNTER_SLOTS:
-            slots.clear()
-        # captures take the slots in turn from the upper half, streams from the lower one
-        half = COUNTER_SLOTS // 2
-        slot = sum((k[0] != 0) == (capture != 0) for k in slots) % half + (half if capture else 0)
-        slots[key] = slot
-    return counters[slot]
+        with torch.cuda.device(device):
+            _lib.check(_lib.kernels().gk_gemm_stream_pool(_lib.ptr(counters), COUNTER_SLOTS, SLOT_INTS), "gemm_stream_pool")
+        _COUNTERS[device.index] = counters
+    return (N + 127) // 128 * 2 <= SLOT_INTS
 
 
 def _linear_f32(x, w, bias, out):
@@ -328,16 +319,18 @@ def linear_forward(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None =
                 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
                 and (out is None or (out.dtype in (torch.bfloat16, torch.float32) and out.stride(1) == 1))
                 and (out is not None or (out_dtype or x.dtype) in (torch.bfloat16, torch.float32))):
-            cnt = _stream_counters(x.device)
-            if cnt is not None:
+            if _stream_ready(x.device, N):
+                lib = _lib.kernels()
                 y = out if out is not None else torch.empty((T, N), dtype=out_dtype or x.dtype, device=x.device)
-                ws = torch.empty(_lib.kernels().gk_gemm_stream_scratch(T), dtype=torch.float32, device=x.device)
+                floats = _STREAM_SCRATCH.get(T)
+                if floats is None:
+                    floats = _STREAM_SCRATCH[T] = lib.gk_gemm_stream_scratch(T)
+                ws = torch.empty(floats, dtype=torch.float32, device=x.device)
                 LAUNCHES["gemm"] += 1
-                rc = _lib.kernels().gk_gemm_stream(
-                    _lib.ptr(w), w.stride(0), _lib.ptr(x), x.stride(0), _lib.ptr(y), y.stride(0),
-                    int(y.dtype == torch.float32), _lib.ptr(bias),
-                    int(bias is not None and bias.dtype == torch.float32), T, N, K, _lib.ptr(ws), ws.numel(),
-                    _lib.ptr(cnt), cnt.numel(), _lib.ptr(_lib.err_flag(x.device)), _lib.stream_ptr())
+                rc = lib.gk_gemm_stream(
+                    w.data_ptr(), w.stride(0), x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0),
+                    y.dtype == torch.float32, _lib.ptr(bias), bias is not None and bias.dtype == torch.float32, T, N, K,
+                    ws.data_ptr(), floats, _lib.err_flag(x.device).data_ptr(), _lib.stream_ptr())
                 _lib.check(rc, "gk_gemm_stream")
                 return y
         bn = 32 if T <= 32 else (64 if T <= 64 else 128)

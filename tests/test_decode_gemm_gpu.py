@@ -37,3 +37,37 @@ def test_stream_gemm(N, K, T):
     assert torch.equal(out, G.linear_forward(x, w, b, out_dtype=torch.float32))
     assert bool((out._base[:, :8] == 7).all()) and bool((out._base[:, N + 8:] == 7).all())
     _lib.check_device_errors()
+
+
+def test_streams_and_captured_branches_keep_their_counters_apart():
+    """Launches that may overlap: four streams at once, and two branches of one graph."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    T, N, K = 8, 3584, 4096
+    g = torch.Generator(device="cuda").manual_seed(3)
+    xs = [torch.randn(T, K, generator=g, device="cuda").bfloat16() for _ in range(4)]
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    ref = [G.linear_forward(x, w, out_dtype=torch.float32) for x in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    torch.cuda.synchronize()
+    outs = [[] for _ in xs]
+    for _ in range(20):
+        for s, x, o in zip(streams, xs, outs):
+            with torch.cuda.stream(s):
+                o.append(G.linear_forward(x, w, out_dtype=torch.float32))
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, r) for o, r in zip(outs, ref) for y in o)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph):
+        side.wait_stream(torch.cuda.current_stream())
+        a = G.linear_forward(xs[0], w, out_dtype=torch.float32)
+        with torch.cuda.stream(side):
+            b = G.linear_forward(xs[1], w, out_dtype=torch.float32)
+        torch.cuda.current_stream().wait_stream(side)
+    for _ in range(5):
+        a.zero_()
+        b.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(a, ref[0]) and torch.equal(b, ref[1])
+    _lib.check_device_errors()
