@@ -22,6 +22,11 @@
 //                         B holds one weight per group stacked along rows.
 //   * ragged-K groups   - MoE wgrad: the contraction runs over each expert's row segment, one C per group.
 //
+// A plain or fp32-accumulated result leaves through shared memory and TMA (32 rows x 128 bytes a copy; sums into C are
+// formed in L2, so that no thread waits for C's old values); other results, and unaligned ones, are stored by the threads.
+// Expert weight gradients are bound by these bytes (us, threads -> TMA, 128 experts of about 281 rows: [1536 x 2048] added
+// to C 1913 -> 839, stored 747 -> 437; [2048 x 768] 989 -> 362, 448 -> 222).
+//
 // Replaces the reference's TileLang `gemm_impl` (gfused/mygemm_fp8.py:13-41) and the cuBLAS/TE GEMMs reached
 // through Megatron-Core.
 #include "ptx.cuh"
@@ -57,6 +62,7 @@ struct GemmParams {
   int* err;
   int stages;   // shared-memory ring depth actually used (<= Cfg::STAGES)
   int group_m;  // tile order of dense problems (host_utils.h: raster_tile)
+  int staged;   // the result leaves through shared memory and TMA
   int a_early;  // operand A does not depend on the kernel before this one (decode: A is the weight): its first
                 // tiles are requested before the programmatic-dependency wait, while the predecessor still runs
 };
@@ -70,6 +76,7 @@ struct Tile {
   long long c_off;  // element offset into C
   int mn_index;     // index of the (m,n) tile for split-K bookkeeping
   int ks;           // split-K slice
+  int group;        // C's plane
 };
 
 template <int BN>
@@ -80,7 +87,8 @@ struct Cfg {
   static constexpr int STAGES_RAW = (192 * 1024) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
   static constexpr int TMEM_COLS = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ +
+  static constexpr int EPI_BYTES = 4 * 32 * 128;   // staging rows of the four epilogue warps
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align*/ + 256 /*barriers*/ +
                                     (MAX_GROUPS + 1) * 4;
 };
 
@@ -96,6 +104,7 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const int* s_pr
   Tile t;
   const int nt = (p.N + BN - 1) / BN;
   t.ks = 0;
+  t.group = 0;
   t.b_y_off = 0;
   t.c_off = 0;
   if (p.group_mode == 1) {
@@ -126,6 +135,7 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const int* s_pr
     t.k0 = p.group_offsets[g];
     t.kblocks = (p.group_offsets[g + 1] - p.group_offsets[g] + BK - 1) / BK;
     t.m_limit = p.M;
+    t.group = g;
     t.c_off = static_cast<long long>(g) * p.c_group_stride;
     t.mn_index = tile;
   } else {
@@ -248,22 +258,92 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const Tile& t, 
   }
 }
 
+// An epilogue warp's 32 rows of a tile through its staging area: 32 fp32 or 64 bf16 columns a TMA copy, 16-byte units
+// XOR-swizzled by row (the tensor map's 128-byte swizzle).  The tensor map clips the ragged edges.
+template <int BN>
+__device__ __forceinline__ void store_tile(const GemmParams& p, const Tile& t, const CUtensorMap& tmC, uint8_t* st,
+                                           uint32_t taddr, int quad, int lane, bool has_acc) {
+  const int row0 = t.m0 + quad * 32;
+#pragma unroll 1
+  for (int c = 0; c < BN / 32; ++c) {
+    const int col0 = t.n0 + c * 32;
+    const bool first = p.out_fp32 || !(c & 1), last = p.out_fp32 || (c & 1);
+    if (first) {
+      if (col0 >= p.N) break;
+      if (lane == 0) tma_store_wait_read();   // the last copy has read the staging rows
+      __syncwarp();
+    }
+    float v[32];
+    if (has_acc) {
+      uint32_t r[32];
+      tmem_ld32(taddr + c * 32, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = 0.f;
+    }
+    if (p.bias && p.bias_along_m) {
+      const int row = row0 + lane;
+      const float b = row >= p.M ? 0.f : p.bias_fp32 ? reinterpret_cast<const float*>(p.bias)[row]
+                                     : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[row]);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] += b;
+    } else if (p.bias) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (col0 + j < p.N)
+          v[j] += p.bias_fp32 ? reinterpret_cast<const float*>(p.bias)[col0 + j]
+                              : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col0 + j]);
+    }
+    if (p.out_fp32) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<float4*>(st + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+            make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint4 o;
+        o.x = pack_bf16x2(v[8 * j + 0], v[8 * j + 1]);
+        o.y = pack_bf16x2(v[8 * j + 2], v[8 * j + 3]);
+        o.z = pack_bf16x2(v[8 * j + 4], v[8 * j + 5]);
+        o.w = pack_bf16x2(v[8 * j + 6], v[8 * j + 7]);
+        *reinterpret_cast<uint4*>(st + lane * 128 + ((((c & 1) * 4 + j) ^ (lane & 7)) << 4)) = o;
+      }
+    }
+    if (last) {
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0 && row0 < p.M) {
+        const int x = p.out_fp32 ? col0 : col0 - 32;
+        if (p.accumulate) tma_reduce_add_3d(&tmC, st, x, row0, t.group);
+        else tma_store_3d(&tmC, st, x, row0, t.group);
+        tma_store_commit();
+      }
+    }
+  }
+}
+
 // MINB = 2 is the decode instantiation: registers are capped so that two CTAs (of this kernel, or this one and the
 // next GEMM of the chain) fit one SM's register file together.
 template <int BN, bool A_MN, bool B_MN, int MINB = 1>
 __global__ void __launch_bounds__(GEMM_THREADS, MINB)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ CUtensorMap tmC, GemmParams p) {
   using C = Cfg<BN>;
   const int STAGES = p.stages;  // ring depth of this launch; the barrier arrays are sized for the maximum
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * C::STAGE_BYTES);
+  uint8_t* epi_stage = smem + STAGES * C::STAGE_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(epi_stage + (p.staged ? C::EPI_BYTES : 0));
   uint64_t* empty = full + C::STAGES;
   uint64_t* tfull = empty + C::STAGES;
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty + 2);
   int* s_flag = reinterpret_cast<int*>(tmem_holder + 1);
-  int* s_prefix = reinterpret_cast<int*>(smem + STAGES * C::STAGE_BYTES + 256);
+  int* s_prefix = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(full) + 256);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -405,6 +485,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       const int row = t.m0 + row_in_tile;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
+      if (MINB == 1 && p.staged) {
+        if (has_acc || !p.accumulate) store_tile<BN>(p, t, tmC, epi_stage + quad * (32 * 128), taddr, quad, lane, has_acc);
+        if (has_acc) {
+          tc_fence_before();
+          mbar_arrive(&tempty[acc]);
+          acc ^= 1;
+          if (acc == 0) pacc ^= 1;
+        }
+        continue;
+      }
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
         float v[32];
@@ -476,6 +566,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         epi_bar_sync();
       }
     }
+    if (MINB == 1 && p.staged && lane == 0) tma_store_wait_all();
   }
 
   tc_fence_before();
@@ -487,7 +578,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 template <int BN, bool A_MN, bool B_MN, int MINB>
-int launch_gemm_q(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& q, int grid, cudaStream_t st) {
+int launch_gemm_q(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const GemmParams& q, int grid,
+                  cudaStream_t st) {
   using C = Cfg<BN>;
   static bool configured = false;
   if (!configured) {
@@ -496,8 +588,8 @@ int launch_gemm_q(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmPara
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
-  const int smem_bytes = q.stages * C::STAGE_BYTES + 1024 + 256 + (MAX_GROUPS + 1) * 4;
-  launch_k(gemm_bf16_kernel<BN, A_MN, B_MN, MINB>, dim3(grid), dim3(GEMM_THREADS), smem_bytes, st, tmA, tmB, q);
+  const int smem_bytes = q.stages * C::STAGE_BYTES + (q.staged ? C::EPI_BYTES : 0) + 1024 + 256 + (MAX_GROUPS + 1) * 4;
+  launch_k(gemm_bf16_kernel<BN, A_MN, B_MN, MINB>, dim3(grid), dim3(GEMM_THREADS), smem_bytes, st, tmA, tmB, tmC, q);
   return launch_status();
 }
 
@@ -505,6 +597,18 @@ template <int BN, bool A_MN, bool B_MN>
 int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int grid, cudaStream_t st) {
   using C = Cfg<BN>;
   GemmParams q = p;
+  // C's planes as a tensor map: one per group of a ragged contraction, else one.  64 bf16 columns a copy need a tile of
+  // whole pairs of 32.  Copies are clipped at 16 bytes, so rows have to be whole multiples of that.
+  const int esz = p.out_fp32 ? 4 : 2;
+  const long long plane = p.group_mode == 2 ? p.c_group_stride : p.ldc * p.M;
+  q.staged = !p.transposed && p.ksplit == 1 && (p.out_fp32 || (!p.accumulate && BN % 64 == 0)) &&
+             (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 && (p.ldc * esz) % 16 == 0 && (plane * esz) % 16 == 0 &&
+             (static_cast<long long>(p.N) * esz) % 16 == 0 &&
+             plane * esz < (1ll << 40);
+  CUtensorMap tmC = tmA;
+  if (q.staged && make_tmap_3d(&tmC, p.C, esz, p.group_mode == 2 ? p.num_groups : 1, p.M, p.N, plane, p.ldc, 1, 32,
+                               128 / esz, true))
+    return -40;
   q.stages = C::STAGES;
   q.a_early = 0;
   q.group_m = gk::raster_group_m();
@@ -518,11 +622,11 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams
         int nst = (decode_smem_cap() - 1024 - 256 - (MAX_GROUPS + 1) * 4) / C::STAGE_BYTES;
         if (nst < 3) nst = 3;
         if (nst < C::STAGES) q.stages = nst;
-        return launch_gemm_q<BN, A_MN, B_MN, 2>(tmA, tmB, q, grid, st);
+        return launch_gemm_q<BN, A_MN, B_MN, 2>(tmA, tmB, tmC, q, grid, st);
       }
     }
   }
-  return launch_gemm_q<BN, A_MN, B_MN, 1>(tmA, tmB, q, grid, st);
+  return launch_gemm_q<BN, A_MN, B_MN, 1>(tmA, tmB, tmC, q, grid, st);
 }
 
 }  // namespace gk

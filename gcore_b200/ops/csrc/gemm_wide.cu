@@ -25,11 +25,12 @@ constexpr int THREADS = 64 + EPI_THREADS;
 constexpr int STAGES = 3;
 constexpr int A_BYTES = BMW * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 // Epilogue staging: every epilogue warp owns 32 rows x 128 bytes (64 bf16 or 32 fp32 columns of its TMEM lane
-// quarter).  Values go from TMEM registers into that area row by row (16-byte units, XOR-swizzled by row so that the
-// 32 lanes of a store hit 32 different banks groups) and leave it as whole 128-byte row segments, four rows per
-// warp-wide store: every global store instruction then writes complete 128-byte lines instead of 32 separate
-// 16-byte fragments.  The accumulators of this kernel are not double-buffered, so the time the epilogue needs to
-// drain the first half of a tile is time the tensor cores wait.
+// quarter).  Values go from TMEM registers into that area row by row (16-byte units, XOR-swizzled by row: no bank
+// conflicts, and the 128-byte swizzle of a tensor map) and leave it as one TMA store, or, where the result is added to
+// C (weight gradients), as one TMA reduction: the addition happens in L2 and no thread waits for C's old values.  The
+// accumulators of this kernel are not double-buffered, so the time the epilogue needs to drain the first half of a tile
+// is time the tensor cores wait.  Measured, us, sums formed by the threads -> in L2: dW [4608 x 3584] over 8000 tokens
+// 259 -> 191, [37888 x 3584] 2029 -> 1439, [3584 x 18944] 1199 -> 810.
 constexpr int MAX_TAIL_KS = 4;      // K-slices of a tail tile (their partials are summed by one CTA)
 constexpr int STAGE_ROW_BYTES = 128;
 constexpr int EPI_STAGE_BYTES = EPI_WARPS * 32 * STAGE_ROW_BYTES;
@@ -45,7 +46,8 @@ struct WParams {
   float alpha;
   int* err;
   int group_m;
-  int staged;   // C rows are 16-byte aligned (and no bf16 read-modify-write): the epilogue stores through shared memory
+  int staged;   // C rows are 16-byte aligned and whole multiples of 16 bytes (copies are clipped at 16 bytes), and no bf16
+                // read-modify-write: the epilogue stores through shared memory
   // Tail split: a problem whose tile count is a little more than a whole number of waves would leave most SMs idle
   // during the last wave (448 tiles on 148 SMs: 3 waves and 4 tiles).  The tiles of that partial wave are cut along K
   // into `tail_ks` slices of `tail_per` k-blocks, each slice is a work item of its own, the slices leave fp32
@@ -141,7 +143,8 @@ __device__ __forceinline__ void store32(const WParams& p, float (&v)[32], int ro
 
 template <bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, WParams p) {
+gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ CUtensorMap tmC, WParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* epi_stage = smem + STAGES * STAGE_BYTES;
@@ -341,6 +344,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           const int row0 = m0 + half * 128 + quad * 32;           // first row of this warp
 #pragma unroll 1
           for (int g0 = chalf * 128; g0 < chalf * 128 + 128; g0 += group_cols) {
+            if (lane == 0) tma_store_wait_read();   // the last copy has read the staging rows
+            __syncwarp();
 #pragma unroll 1
             for (int c = g0 / 32; c < (g0 + group_cols) / 32; ++c) {
               float v[32];
@@ -381,40 +386,13 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 }
               }
             }
+            fence_proxy_async();
             __syncwarp();
-            // drain: lane -> (row 4 i + lane / 8, unit lane % 8); one instruction = four rows x 128 bytes
-            const int unit = lane & 7;
-            const int ucols = 16 / esz;
-            const int col = n0 + g0 + unit * ucols;
-#pragma unroll 4
-            for (int i = 0; i < 8; ++i) {
-              const int rr = 4 * i + (lane >> 3);
-              const int grow = row0 + rr;
-              const uint4 w = *reinterpret_cast<const uint4*>(st + rr * STAGE_ROW_BYTES + ((unit ^ (rr & 7)) << 4));
-              if (grow >= p.M || col >= p.N) continue;
-              uint8_t* dst = reinterpret_cast<uint8_t*>(p.C) + (static_cast<long long>(grow) * p.ldc + col) * esz;
-              if (col + ucols <= p.N) {
-                if (p.out_fp32 && p.accumulate) {
-                  const float4 c4 = *reinterpret_cast<const float4*>(dst);
-                  float4 o = *reinterpret_cast<const float4*>(&w);
-                  o.x += c4.x; o.y += c4.y; o.z += c4.z; o.w += c4.w;
-                  *reinterpret_cast<float4*>(dst) = o;
-                } else {
-                  *reinterpret_cast<uint4*>(dst) = w;
-                }
-              } else if (p.out_fp32) {
-                const float* e = reinterpret_cast<const float*>(&w);
-                float* d = reinterpret_cast<float*>(dst);
-                for (int j = 0; j < ucols; ++j)
-                  if (col + j < p.N) d[j] = p.accumulate ? d[j] + e[j] : e[j];
-              } else {
-                const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&w);
-                __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(dst);
-                for (int j = 0; j < ucols; ++j)
-                  if (col + j < p.N) d[j] = e[j];
-              }
+            if (lane == 0 && row0 < p.M && n0 + g0 < p.N) {   // the tensor map clips the ragged edges
+              if (p.accumulate) tma_reduce_add_2d(&tmC, st, n0 + g0, row0);
+              else tma_store_2d(&tmC, st, n0 + g0, row0);
+              tma_store_commit();
             }
-            __syncwarp();   // the staging rows are free for the next pass
           }
         } else {
 #pragma unroll 1
@@ -438,6 +416,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       pt ^= 1;
     }
+    if (p.staged && lane == 0) tma_store_wait_all();
   }
   tc_fence_before();
   __syncthreads();
@@ -445,7 +424,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 template <bool A_MN, bool B_MN>
-int launch_wide(const CUtensorMap& tmA, const CUtensorMap& tmB, const WParams& p, int grid, cudaStream_t st) {
+int launch_wide(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const WParams& p, int grid,
+                cudaStream_t st) {
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(gemm_wide_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
@@ -453,7 +433,7 @@ int launch_wide(const CUtensorMap& tmA, const CUtensorMap& tmB, const WParams& p
       return -6;
     configured = true;
   }
-  launch_k(gemm_wide_kernel<A_MN, B_MN>, dim3(grid), dim3(THREADS), SMEM_BYTES, st, tmA, tmB, p);
+  launch_k(gemm_wide_kernel<A_MN, B_MN>, dim3(grid), dim3(THREADS), SMEM_BYTES, st, tmA, tmB, tmC, p);
   return launch_status();
 }
 
@@ -487,8 +467,11 @@ GK_EXPORT int gk_gemm_wide(const void* A, long long lda, long long a_rows, int a
   p.bias = bias; p.bias_fp32 = bias_fp32; p.alpha = alpha; p.err = err;
   p.group_m = gk::raster_group_m();
   const int esz = out_fp32 ? 4 : 2;
-  p.staged = ((reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc * esz) % 16 == 0 && (out_fp32 || !accumulate) &&
+  p.staged = ((reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc * esz) % 16 == 0 && (static_cast<long long>(N) * esz) % 16 == 0 &&
+              (out_fp32 || !accumulate) &&
               gk::wide_staged_epilogue()) ? 1 : 0;
+  CUtensorMap tmC = tmA;
+  if (p.staged && gk::make_tmap_2d(&tmC, C, esz, M, N, ldc, 32, STAGE_ROW_BYTES / esz, true)) return -40;
   const long long tiles = static_cast<long long>((M + BMW - 1) / BMW) * ((N + BN - 1) / BN);
   const int sms = gk::sm_count();
   int grid = static_cast<int>(tiles < sms ? tiles : sms);
@@ -510,8 +493,8 @@ GK_EXPORT int gk_gemm_wide(const void* A, long long lda, long long a_rows, int a
     }
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (!a_mn && !b_mn) return launch_wide<false, false>(tmA, tmB, p, grid, st);
-  if (a_mn && !b_mn) return launch_wide<true, false>(tmA, tmB, p, grid, st);
-  if (!a_mn && b_mn) return launch_wide<false, true>(tmA, tmB, p, grid, st);
-  return launch_wide<true, true>(tmA, tmB, p, grid, st);
+  if (!a_mn && !b_mn) return launch_wide<false, false>(tmA, tmB, tmC, p, grid, st);
+  if (a_mn && !b_mn) return launch_wide<true, false>(tmA, tmB, tmC, p, grid, st);
+  if (!a_mn && b_mn) return launch_wide<false, true>(tmA, tmB, tmC, p, grid, st);
+  return launch_wide<true, true>(tmA, tmB, tmC, p, grid, st);
 }
