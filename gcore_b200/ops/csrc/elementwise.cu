@@ -310,39 +310,108 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const 
 // One pass over the optimizer shard: unscale/clip the gradient, AdamW on the fp32 master, write the bf16
 // parameter.  `scale_ptr` (device) holds the combined gradient multiplier (1/loss-scale * clip coefficient) so
 // the clip coefficient never visits the host.
-__global__ void adam_kernel(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
-                            const void* __restrict__ grad, int grad_fp32, __nv_bfloat16* __restrict__ param,
-                            long long n, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2,
-                            const float* __restrict__ scale_ptr, float scale_val) {
-  const float scale = (scale_ptr ? *scale_ptr : 1.f) * scale_val;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float g = (grad_fp32 ? reinterpret_cast<const float*>(grad)[i]
-                               : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(grad)[i])) * scale;
-    const float mi = b1 * m[i] + (1.f - b1) * g;
-    const float vi = b2 * v[i] + (1.f - b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    float p = master[i];
-    const float upd = (mi / bc1) / (sqrtf(vi / bc2) + eps) + wd * p;
-    p -= lr * upd;
-    master[i] = p;
-    if (param) param[i] = __float2bfloat16(p);
+struct AdamArgs {
+  float *master, *m, *v;
+  const void* grad;
+  __nv_bfloat16* param;   // or null
+  long long n;
+  float lr, b1, b2, eps, wd, bc1, bc2;
+  const float* scale_ptr;
+  float scale_val;
+};
+__device__ __forceinline__ float adam_one(const AdamArgs& a, float g, float& m, float& v, float p) {
+  m = a.b1 * m + (1.f - a.b1) * g;
+  v = a.b2 * v + (1.f - a.b2) * g * g;
+  const float upd = (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps) + a.wd * p;
+  return p - a.lr * upd;
+}
+// HBM-bound at 28 bytes moved per element (fp32 gradient).  VEC: a thread takes four neighbours at a time, so that it has
+// 64 bytes in flight instead of 16 (700 M elements: 3.62 ms, 5.4 TB/s, against 4.69 ms; 45 M: 241 against 291 us).  The scalar form serves unaligned shards and the last elements.
+template <bool GRAD32, bool VEC>
+__global__ void __launch_bounds__(256) adam_kernel(const AdamArgs a, long long first) {
+  const float scale = (a.scale_ptr ? *a.scale_ptr : 1.f) * a.scale_val;
+  const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  if (VEC) {
+    for (long long i = t * 4; i + 3 < a.n; i += step * 4) {
+      float4 g;
+      if (GRAD32) {
+        g = __ldcs(reinterpret_cast<const float4*>(static_cast<const float*>(a.grad) + i));
+      } else {
+        const uint2 r = __ldcs(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(a.grad) + i));
+        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
+        const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
+        g = make_float4(x.x, x.y, y.x, y.y);
+      }
+      float4 m = __ldcs(reinterpret_cast<const float4*>(a.m + i)), v = __ldcs(reinterpret_cast<const float4*>(a.v + i));
+      float4 p = __ldcs(reinterpret_cast<const float4*>(a.master + i));
+      p.x = adam_one(a, g.x * scale, m.x, v.x, p.x);
+      p.y = adam_one(a, g.y * scale, m.y, v.y, p.y);
+      p.z = adam_one(a, g.z * scale, m.z, v.z, p.z);
+      p.w = adam_one(a, g.w * scale, m.w, v.w, p.w);
+      __stcs(reinterpret_cast<float4*>(a.m + i), m);
+      __stcs(reinterpret_cast<float4*>(a.v + i), v);
+      __stcs(reinterpret_cast<float4*>(a.master + i), p);
+      if (a.param) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(p.x, p.y), hi = __floats2bfloat162_rn(p.z, p.w);
+        uint2 r;
+        r.x = *reinterpret_cast<const uint32_t*>(&lo);
+        r.y = *reinterpret_cast<const uint32_t*>(&hi);
+        *reinterpret_cast<uint2*>(a.param + i) = r;
+      }
+    }
+  } else {
+    for (long long i = first + t; i < a.n; i += step) {
+      const float g = (GRAD32 ? static_cast<const float*>(a.grad)[i]
+                              : __bfloat162float(static_cast<const __nv_bfloat16*>(a.grad)[i])) * scale;
+      float m = a.m[i], v = a.v[i];
+      const float p = adam_one(a, g, m, v, a.master[i]);
+      a.m[i] = m;
+      a.v[i] = v;
+      a.master[i] = p;
+      if (a.param) a.param[i] = __float2bfloat16(p);
+    }
   }
 }
 
-__global__ void __launch_bounds__(256) sumsq_kernel(const void* __restrict__ x, int is_fp32, long long n,
-                                                    float* __restrict__ out) {
+// Every thread keeps four partial sums, over elements `first` and on; VEC (16-byte aligned input): 16 bytes a load, four
+// loads in flight (700 M fp32: 468 us, 6.0 TB/s, against 729 us; 45 M: 47 against 64 us).
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256) sumsq_kernel(const T* __restrict__ x, long long n, float* __restrict__ out) {
   __shared__ float red[32];
-  float s = 0.f;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float f = is_fp32 ? reinterpret_cast<const float*>(x)[i]
-                            : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(x)[i]);
-    s += f * f;
+  constexpr int W = 16 / sizeof(T);
+  const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  long long done = 0;
+  if (VEC) {
+    const long long nv = n / W;
+    const uint4* xv = reinterpret_cast<const uint4*>(x);
+    auto add = [](uint4 r, float& acc) {
+      const T* e = reinterpret_cast<const T*>(&r);
+#pragma unroll
+      for (int j = 0; j < W; ++j) {
+        const float f = static_cast<float>(e[j]);
+        acc += f * f;
+      }
+    };
+    long long i = t;
+    for (; i + 3 * step < nv; i += 4 * step) {
+      uint4 r[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) r[u] = __ldg(xv + i + u * step);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) add(r[u], s[u]);
+    }
+    for (; i < nv; i += step) add(__ldg(xv + i), s[0]);
+    done = nv * W;
   }
-  s = block_sum(s, red);
-  if (threadIdx.x == 0) atomicAdd(out, s);
+  for (long long i = done + t; i < n; i += step) {
+    const float f = static_cast<float>(x[i]);
+    s[1] += f * f;
+  }
+  const float sum = block_sum((s[0] + s[1]) + (s[2] + s[3]), red);
+  if (threadIdx.x == 0) atomicAdd(out, sum);
 }
 
 // dst(bf16 or fp32) (+)= scale * src
@@ -506,16 +575,42 @@ GK_EXPORT int gk_adam(float* master, float* m, float* v, const void* grad, int g
   if (n == 0) return 0;
   const float bc1 = 1.f - powf(b1, static_cast<float>(step));
   const float bc2 = 1.f - powf(b2, static_cast<float>(step));
-  adam_kernel<<<grid_for(n, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      master, m, v, grad, grad_fp32, reinterpret_cast<__nv_bfloat16*>(param), n, lr, b1, b2, eps, wd, bc1, bc2,
-      scale_ptr, scale_val);
+  const AdamArgs a = {master, m, v, grad, reinterpret_cast<__nv_bfloat16*>(param), n, lr, b1, b2, eps, wd, bc1, bc2,
+                      scale_ptr, scale_val};
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  auto bits = [](const void* p) { return reinterpret_cast<uintptr_t>(p); };
+  const bool vec = ((bits(master) | bits(m) | bits(v) | (grad_fp32 ? bits(grad) : 0)) & 15) == 0 &&
+                   ((bits(param) | bits(grad)) & 7) == 0;
+  long long first = 0;
+  if (vec && n >= 4) {
+    first = n / 4 * 4;
+    const int grid = grid_for(n / 4, 256);
+    if (grad_fp32) adam_kernel<true, true><<<grid, 256, 0, st>>>(a, 0);
+    else adam_kernel<false, true><<<grid, 256, 0, st>>>(a, 0);
+  }
+  if (first < n) {
+    const int grid = grid_for(n - first, 256);
+    if (grad_fp32) adam_kernel<true, false><<<grid, 256, 0, st>>>(a, first);
+    else adam_kernel<false, false><<<grid, 256, 0, st>>>(a, first);
+  }
   return launch_status();
 }
 
 // out[0] += sum(x^2); the caller zeroes out[0].
 GK_EXPORT int gk_sumsq(const void* x, int is_fp32, long long n, float* out, void* stream) {
   if (n == 0) return 0;
-  sumsq_kernel<<<grid_for(n, 256, 4), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(x, is_fp32, n, out);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const int grid = grid_for(n, 256 * (vec ? 16 : 1), 8);
+  if (is_fp32) {
+    const float* f = static_cast<const float*>(x);
+    if (vec) sumsq_kernel<float, true><<<grid, 256, 0, st>>>(f, n, out);
+    else sumsq_kernel<float, false><<<grid, 256, 0, st>>>(f, n, out);
+  } else {
+    const __nv_bfloat16* h = static_cast<const __nv_bfloat16*>(x);
+    if (vec) sumsq_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(h, n, out);
+    else sumsq_kernel<__nv_bfloat16, false><<<grid, 256, 0, st>>>(h, n, out);
+  }
   return launch_status();
 }
 
