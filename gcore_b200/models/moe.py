@@ -14,7 +14,7 @@ import torch
 import torch.nn as nn
 
 from ..core import parallel_state as ps
-from ..ops import fused
+from ..ops import _lib, fused, moe as moe_ops
 from ..ops.gemm import grouped_gemm, grouped_wgrad
 from .config import ModelConfig
 
@@ -271,14 +271,56 @@ class MoELayer(nn.Module):
             self.shared_expert_gate.weight.tp_mode = "none"
             self.shared_expert_gate.weight.sequence_parallel = True
 
+    def _native(self, x) -> bool:
+        """Whether tokens move to plain bf16 experts and back through the fused kernels."""
+        e = self.experts
+        return (self.ep_size == 1 and _lib.use_native(x) and x.dtype == torch.bfloat16 and x.shape[0] > 0
+                and x.shape[1] % 8 == 0 and self.cfg.num_experts <= moe_ops.MAX_EXPERTS and e.precision is None
+                and e.lora_fc1 is None and e.lora_fc2 is None and e.linear_fc1.weight.dtype == torch.bfloat16)
+
+    def _decode_ready(self, x) -> bool:
+        """Whether the layer runs on the decode kernels: up to 128 tokens an expert has a few, and their 16-row segments read
+        its weights about once (128 experts, top 8: 128 tokens 232 us, 256 through the general kernels 381; the routing
+        kernel's logits are built for as many)."""
+        cfg, r, e = self.cfg, self.router, self.experts
+        E, K = cfg.num_experts, cfg.moe_top_k
+        sigmoid = cfg.moe_router_type != "softmax"
+        return (not self.training and not torch.is_grad_enabled() and x.shape[0] <= moe_ops.DECODE_TOKENS
+                and x.shape[1] <= moe_ops.DECODE_WIDTH and cfg.moe_ffn_hidden_size % 64 == 0 and E in (32, 64, 128, 256, 512)
+                and 1 <= K <= min(moe_ops.MAX_TOP, E) and (not sigmoid or (1 <= cfg.moe_n_group <= 8 and E % cfg.moe_n_group == 0))
+                and RouterReplay.mode != "replay" and r.lora is None and r.weight.dtype == torch.float32
+                and all(t.is_contiguous() and t.data_ptr() % 16 == 0
+                        for t in (r.weight, e.linear_fc1.weight, e.linear_fc2.weight)))
+
+    def _decode(self, x):
+        cfg, r = self.cfg, self.router
+        sigmoid = cfg.moe_router_type != "softmax"
+        y, idx = moe_ops.decode_layer(
+            x, r.weight, r.expert_bias.float() if sigmoid and r.expert_bias is not None else None,
+            self.experts.linear_fc1.weight, self.experts.linear_fc2.weight, cfg.moe_top_k, sigmoid, cfg.moe_norm_topk_prob,
+            cfg.moe_routed_scaling_factor if sigmoid else 1.0, cfg.moe_n_group if sigmoid else 1,
+            cfg.moe_topk_group if sigmoid else 1)
+        if RouterReplay.mode == "record":
+            RouterReplay.put(r.layer_idx, idx)
+        return y
+
     def forward(self, x):
         cfg = self.cfg
         T, H = x.shape
         K = cfg.moe_top_k
+        native = self._native(x)
+        if native and not (x.is_contiguous() and x.data_ptr() % 16 == 0):
+            x = x.clone(memory_format=torch.contiguous_format)
+        if native and self._decode_ready(x):
+            return self._add_shared(x, self._decode(x)), None
         idx, w, aux = self.router(x)
         if self.ep_size > 1:
             from ..parallel.ep import ep_moe_forward
             y = ep_moe_forward(self, x, idx, w)
+        elif native:
+            dest, src, offsets = moe_ops.plan_rows(idx.contiguous(), cfg.num_experts)
+            y_perm = self.experts(moe_ops.GatherRows.apply(x, dest, src, offsets), offsets)
+            y = moe_ops.CombineRows.apply(y_perm, w.float().contiguous(), dest, src, offsets)
         else:
             flat_e = idx.reshape(-1)
             dest, offsets = build_dispatch_plan(flat_e, cfg.num_experts)
@@ -288,9 +330,12 @@ class MoELayer(nn.Module):
             x_perm = x_perm.index_copy(0, dest, x[token_of])
             y_perm = self.experts(x_perm, offsets)
             y = (y_perm[dest].view(T, K, H) * w.to(x.dtype)[:, :, None]).sum(1)
+        return self._add_shared(x, y), aux
+
+    def _add_shared(self, x, y):
         if self.shared_experts is not None:
             ys = self.shared_experts(x)
             if self.shared_expert_gate is not None:
                 ys = ys * torch.sigmoid(torch.nn.functional.linear(x, self.shared_expert_gate.weight))
             y = y + ys
-        return y, aux
+        return y

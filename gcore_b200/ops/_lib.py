@@ -230,7 +230,14 @@ def _declare_kernels(lib: ctypes.CDLL):
     d("gk_memory_output", [I, P, P, L, P, P, L, P, F, F, P])
     d("gk_depth_average", [I, P, L, P, F, P])
     d("gk_ffn_act", [I, I, P, P, P, P])
-    d("gk_expert_rows", [P, P, P, P, P, P, P, I, I, I, I, P])
+    d("gk_expert_rows", [P, P, P, P, P, P, P, I, I, I, I, I, P])
+    d("gk_moe_plan_scratch", [I, I], L)
+    d("gk_moe_plan", [P, I, I, I, P, P, P, P, P])
+    d("gk_moe_gather", [P, P, P, P, I, I, I, P])
+    d("gk_moe_combine", [P, P, P, P, I, I, I, P])
+    d("gk_moe_combine_bwd", [P, P, P, P, P, P, P, I, I, I, P])
+    d("gk_router_logits", [P, P, P, P, I, I, I, P])
+    d("gk_moe_decode", [P, P, P, P, P, I, I, I, I, I, P, P])
     d("gk_grouped_gemm_f32", [P, P, P, P, I, I, I, I, P])
     d("gk_router_dispatch", [P, L, P, P, P, P, P, L, I, I, I, I, F, I, I, P])
     d("gk_router_fused", [I, P, P, P, I, I, P, P, P, P, P, L, I, I, I, I, F, I, I, P])

@@ -375,13 +375,20 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     prefetch_tmap(&tmB);
     if (!p.a_early) prefetch_tmap(&tmA);
   }
-  if (threadIdx.x == 32 && p.group_mode == 1) {
+  if (warp == 1 && p.group_mode == 1) {
     pdl_wait();  // the group offsets come from the kernel before this one
     int acc = 0;
-    s_prefix[0] = 0;
-    for (int g = 0; g < p.num_groups; ++g) {
-      acc += (p.group_offsets[g + 1] - p.group_offsets[g] + BM - 1) / BM;
-      s_prefix[g + 1] = acc;
+    if (lane == 0) s_prefix[0] = 0;
+    for (int g0 = 0; g0 < p.num_groups; g0 += 32) {   // 32 groups at a time
+      const int g = g0 + lane;
+      int v = g < p.num_groups ? (p.group_offsets[g + 1] - p.group_offsets[g] + BM - 1) / BM : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
+      }
+      if (g < p.num_groups) s_prefix[g + 1] = acc + v;
+      acc += __shfl_sync(0xffffffffu, v, 31);
     }
   }
   if (warp == 2) {

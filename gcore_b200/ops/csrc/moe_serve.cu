@@ -2,7 +2,7 @@
 // around the grouped GEMMs when routing has counted the tokens of every expert (router.cu):
 //   * ffn_act_kernel        silu(gate) * up or relu(up)^2, optionally scaled by a sigmoid per row, between two strided
 //                           matrices;
-//   * expert_rows_kernel    segment offsets (128-row segments, as the grouped GEMM wants them) and the copy of every
+//   * expert_rows_kernel    segment offsets (segments of 128 or 16 rows, as the grouped GEMMs want them) and the copy of every
 //                           token's row into its experts' segments, one launch;
 //   * grouped_f32_kernel    the grouped product in true 32-bit, for models that run in 32-bit.
 #include "host_utils.h"
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(ER_THREADS) expert_rows_kernel(const uint4* __
                                                                  const long long* __restrict__ choice,
                                                                  const int* __restrict__ place, int* __restrict__ offsets,
                                                                  int* __restrict__ dest, uint4* __restrict__ out,
-                                                                 int n, int K, int E, int row_vec) {
+                                                                 int n, int K, int E, int seg, int row_vec) {
   __shared__ int s_off[ER_MAX_EXPERTS + 1];
   __shared__ int s_warp[ER_THREADS / 32];
   pdl_launch_dependents();
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(ER_THREADS) expert_rows_kernel(const uint4* __
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // exclusive prefix sums of the padded counts: two experts per thread
   const int e0 = 2 * tid;
-  const int a = e0 < E ? (counts[e0] + 127) / 128 * 128 : 0, b = e0 + 1 < E ? (counts[e0 + 1] + 127) / 128 * 128 : 0;
+  const int a = e0 < E ? (counts[e0] + seg - 1) / seg * seg : 0, b = e0 + 1 < E ? (counts[e0 + 1] + seg - 1) / seg * seg : 0;
   int incl = a + b;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -188,16 +188,16 @@ GK_EXPORT int gk_ffn_act(int act, int is_fp32, void* const* ptrs, const long lon
   return is_fp32 ? fill(static_cast<float*>(nullptr)) : fill(static_cast<__nv_bfloat16*>(nullptr));
 }
 
-// choice, place: [tokens * K]; out: room for every token's rows with the segments padded to 128.  row_bytes % 16 == 0.
+// choice, place: [tokens * K]; out: room for every token's rows with the segments padded to `seg`.  row_bytes % 16 == 0.
 GK_EXPORT int gk_expert_rows(const void* h, const int* counts, const long long* choice, const int* place, int* offsets,
-                             int* dest, void* out, int tokens, int K, int E, int row_bytes, void* stream) {
-  if (E < 1 || E > ER_MAX_EXPERTS || K < 1 || row_bytes % 16) return -1;
+                             int* dest, void* out, int tokens, int K, int E, int seg, int row_bytes, void* stream) {
+  if (seg < 1 || E < 1 || E > ER_MAX_EXPERTS || K < 1 || row_bytes % 16) return -1;
   const int n = tokens * K;
   int blocks = (n + ER_THREADS / 32 - 1) / (ER_THREADS / 32);
   if (blocks > sm_count() * 8) blocks = sm_count() * 8;
   if (blocks < 1) blocks = 1;
   launch_k(expert_rows_kernel, dim3(blocks), dim3(ER_THREADS), 0, reinterpret_cast<cudaStream_t>(stream),
-           static_cast<const uint4*>(h), counts, choice, place, offsets, dest, static_cast<uint4*>(out), n, K, E,
+           static_cast<const uint4*>(h), counts, choice, place, offsets, dest, static_cast<uint4*>(out), n, K, E, seg,
            row_bytes / 16);
   return launch_status();
 }
