@@ -2,6 +2,8 @@
 add, RoPE, SwiGLU.  Each has a plain PyTorch implementation used on CPU and as the test oracle."""
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib
@@ -227,3 +229,33 @@ def swiglu(x: torch.Tensor, n_rows: torch.Tensor = None) -> torch.Tensor:
             return out
         return _SwigluFn.apply(x)
     return swiglu_ref(x)
+
+
+def decode_begin(st, block: int, embed=None, sink=None):
+    """In front of a decode step over the batch state ``st`` (GPU tensors): ``(slots, ctx, states, sink_slots, x)``, the cache
+    row of every request's token (-1 where nothing is stored: a row that rests or has reached its limit), the tokens it sees,
+    its recurrent state's slot or -1, with ``sink`` the rows once more with ``sink`` for -1 (int64), and with ``embed`` the
+    tokens' embedding rows."""
+    B, max_blocks = st["block_table"].shape
+    dev = st["pos"].device
+    slots, ctx, states = (torch.empty(B, dtype=torch.int32, device=dev) for _ in range(3))
+    sink_slots = torch.empty(B, dtype=torch.int64, device=dev) if sink is not None else None
+    x = torch.empty(B, embed.shape[1], dtype=embed.dtype, device=dev) if embed is not None else None
+    ptrs = (ctypes.c_void_p * 12)(*[t.data_ptr() if t is not None else None for t in (
+        st["tokens"], st["pos"], st["active"], st["limit"], st["block_table"], st["state"], embed, slots, ctx, states,
+        sink_slots, x)])
+    dims = (ctypes.c_longlong * 6)(B, max_blocks, block, embed.shape[1] * embed.element_size() if embed is not None else 0,
+                                   embed.shape[0] if embed is not None else 0, sink if sink is not None else 0)
+    LAUNCHES["elementwise"] += 1
+    _lib.check(_lib.kernels().gk_decode_begin(ptrs, dims, _lib.stream_ptr()), "decode_begin")
+    return slots, ctx, states, sink_slots, x
+
+
+def decode_end(st, tok, lp):
+    """Behind a decode step: the drawn tokens into the batch state and, with their log-probs, into the output ring; active
+    rows advance."""
+    ptrs = (ctypes.c_void_p * 9)(*[t.data_ptr() for t in (tok, lp, st["active"], st["tokens"], st["pos"], st["steps"],
+                                                         st["ring_idx"], st["ring_tok"], st["ring_lp"])])
+    LAUNCHES["elementwise"] += 1
+    _lib.check(_lib.kernels().gk_decode_end(ptrs, st["tokens"].numel(), st["ring_tok"].shape[0], _lib.stream_ptr()),
+               "decode_end")

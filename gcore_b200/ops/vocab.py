@@ -239,7 +239,8 @@ def sample(logits, temperature, seeds, steps, greedy=False, tp_group=None, vocab
     tp = dist.get_world_size(tp_group) if tp_group is not None else 1
     # a row of a large vocabulary is shared by several CTAs (the random stream is evaluated per element: one CTA per
     # row leaves most of the GPU idle at decode batch sizes); their partials merge like tensor-parallel shards
-    slices = max(1, min(8, 592 // max(B, 1))) if V >= 16384 else 1
+    # (four CTAs on each of 148 SMs, slices of at least 2048)
+    slices = max(1, min(32, 592 // max(B, 1), V // 2048)) if V >= 16384 else 1
     LAUNCHES["vocab"] += 1
     if tp == 1 and slices == 1:
         _lib.check(lib.gk_sample(_lib.ptr(logits), int(logits.dtype == torch.float32), logits.stride(0), V, vocab_start,

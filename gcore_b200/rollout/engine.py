@@ -630,23 +630,33 @@ class InferEngine:
         cfg = self.cfg
         B = st["tokens"].numel()
         pos = st["pos"]
-        blk = st["block_table"].gather(1, (pos // self.bs).long()[:, None].clamp_max(self.max_blocks - 1)).squeeze(1)
-        # a request at its length limit has no cache behind it: the rest of the interval is discarded, nothing is stored
-        live = st["active"] & (pos < st["limit"])
-        slots = torch.where(live, blk * self.bs + pos % self.bs, torch.full_like(pos, -1))
-        ctx = torch.where(live, pos + 1, torch.zeros_like(pos))
+        sink = (self.k_cache[0].shape[0] - 1) * self.bs if self.mla_dim else None
+        native = self._native_state()
+        x = lat_slots = None
+        if native:
+            own = self.plan is None and self.tp == 1 and self.w.embed.is_contiguous() and self.w.embed.data_ptr() % 16 == 0 \
+                and self.w.embed.shape[1] * self.w.embed.element_size() % 16 == 0
+            slots, ctx, states, lat_slots, x = fused.decode_begin(st, self.bs, self.w.embed if own else None, sink)
+        else:
+            blk = st["block_table"].gather(1, (pos // self.bs).long()[:, None].clamp_max(self.max_blocks - 1)).squeeze(1)
+            # a request at its length limit has no cache behind it: the rest of the interval is discarded, nothing is stored
+            live = st["active"] & (pos < st["limit"])
+            slots = torch.where(live, blk * self.bs + pos % self.bs, torch.full_like(pos, -1))
+            ctx = torch.where(live, pos + 1, torch.zeros_like(pos))
+            states = torch.where(live, st["state"], torch.full_like(pos, -1))
         if self.plan is not None:
             rows = StepRows(tokens=st["tokens"], pos=pos, slots=slots, tables=st["block_table"],
-                            states=torch.where(live, st["state"], torch.full_like(pos, -1)), first_pos=pos, cu=None,
+                            states=states, first_pos=pos, cu=None,
                             ctx=ctx, row_seq=st["row_seq"], n_portions=0, portion_rows=0, max_portion=0,
                             max_ctx=self.max_model_len)
             self._finish_decode(self.plan(rows, self.k_cache, self.memory), st)
             return
-        x = self._embed(st["tokens"])
+        if x is None:
+            x = self._embed(st["tokens"])
         res = None
         if self.mla_dim:
-            sink = (self.k_cache[0].shape[0] - 1) * self.bs
-            lat_slots = torch.where(slots >= 0, slots, torch.full_like(slots, sink)).long()
+            if lat_slots is None:
+                lat_slots = torch.where(slots >= 0, slots, torch.full_like(slots, sink)).long()
             lat_idx = lat_mask = None
             if not self._mla_native():
                 # eager form: latent rows of every request, gathered once per step for all layers' index arithmetic
@@ -676,10 +686,20 @@ class InferEngine:
 
     def _finish_decode(self, hl, st):
         """Samples the next token of every row and advances the batch state."""
-        self._sample_into(hl, st)
+        tok, lp = self._draw(hl, st)
+        if st["params"].get("repetition_penalty", 1.0) != 1.0:
+            st["seen"].scatter_(1, tok[:, None], True)
+        if self._native_state():
+            fused.decode_end(st, tok, lp)
+            return
+        self._store_drawn(tok, lp, st)
         st["pos"].add_(st["active"].to(st["pos"].dtype))
         st["steps"].add_(1)
         st["ring_idx"].add_(1)
+
+    def _native_state(self) -> bool:
+        """Whether the batch state of a decode step is advanced by kernels."""
+        return self.device.type == "cuda" and not _lib.force_eager() and hasattr(_lib.kernels(), "gk_decode_begin")
 
     def _ep_any(self, *flags):
         """Logical OR of each flag over the engines of the expert-parallel group (one small all-reduce)."""
@@ -775,7 +795,8 @@ class InferEngine:
         o = torch.einsum("bhc,hvc->bhv", o_lat, w_up[:, dn:].float())
         return o.reshape(B, mla.h * dv).to(h.dtype)
 
-    def _sample_into(self, hidden, st):
+    def _draw(self, hidden, st):
+        """The next token of every row and its log-prob."""
         logits = linear_forward(hidden, self.w.head, out_dtype=torch.float32)
         sp = st["params"]
         penalise = sp.get("repetition_penalty", 1.0) != 1.0
@@ -797,9 +818,11 @@ class InferEngine:
         else:
             tok, lp = sample(logits, sp["temperature"], st["seeds"], st["steps"], sp["greedy"],
                              self.tp_group if self.tp > 1 else None, self.vocab_start)
+        return tok, lp
+
+    @staticmethod
+    def _store_drawn(tok, lp, st):
         st["tokens"].copy_(tok)
-        if penalise:
-            st["seen"].scatter_(1, tok[:, None], True)
         idx = st["ring_idx"] % st["ring_tok"].shape[0]
         st["ring_tok"].index_copy_(0, idx, tok[None])
         st["ring_lp"].index_copy_(0, idx, lp[None])
@@ -1137,17 +1160,13 @@ class InferEngine:
                         owners.append(c)
                 hsel = hl[torch.tensor(rows, device=dev)]
                 sd = torch.tensor([c.seed for c in owners], dtype=torch.int64, device=dev)
-                tmp = dict(tokens=torch.zeros(len(owners), dtype=torch.int64, device=dev), seeds=sd,
-                           steps=torch.zeros(len(owners), dtype=torch.int32, device=dev),
-                           ring_tok=torch.zeros(1, len(owners), dtype=torch.int64, device=dev),
-                           ring_lp=torch.zeros(1, len(owners), dtype=torch.float32, device=dev),
-                           ring_idx=torch.zeros(1, dtype=torch.int64, device=dev), params=st["params"])
+                tmp = dict(seeds=sd, steps=torch.zeros(len(owners), dtype=torch.int32, device=dev), params=st["params"])
                 if "seen" in st:
                     tmp["seen"] = torch.zeros(len(owners), self._vocab_total(), dtype=torch.bool, device=dev)
                     for k, c in enumerate(owners):
                         tmp["seen"][k, torch.tensor(c.prompt, dtype=torch.int64, device=dev)] = True
-                self._sample_into(hsel, tmp)
-                ft, fl = tmp["ring_tok"][0].tolist(), tmp["ring_lp"][0].tolist()
+                tok, lp = self._draw(hsel, tmp)
+                ft, fl = tok.tolist(), lp.tolist()
                 io_counters.add_d2h(12 * len(owners))
                 first = {c.rid: (t, l) for c, t, l in zip(owners, ft, fl)}
                 # fork the samples before anything of the group can finish, then enter the decode batch
