@@ -50,7 +50,14 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 // ------------------------------------------------------------------------------------------ RMSNorm
-// y = (x [+ res]) * rstd * w ; optionally writes the summed residual stream to res_out.
+// y = (x [+ res]) * rstd * w ; optionally writes the summed residual stream to res_out.  Rows stay in registers between the
+// sum of squares and the scaling, and the gains (weights of the model, which no kernel of a decode chain writes) are read
+// before the wait for the kernel in front.  Every kernel adds the squares in the same order (thread, warp, block), so that a row
+// gives the same bits in each.  us, forward with residual / backward, before -> now: 8000 x 3584 62 / 144 -> 53 / 102, 26000 x
+// 4096 195 / 352 -> 154 / 192, 140000 heads of 128 217 / 633 -> 37 / 82 (calls of less than 80 us backward are host-bound).
+//
+// Rows of more than 256 values: a CTA per row, SLOTS 16-byte units per thread.
+template <int SLOTS>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                           const __nv_bfloat16* __restrict__ res,
                                                           const __nv_bfloat16* __restrict__ w,
@@ -59,56 +66,158 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
                                                           float* __restrict__ rstd_out, int T, int H, float eps) {
   __shared__ float red[32];
   pdl_launch_dependents();
+  const int nv = H >> 3;
+  bf16x8 gain[SLOTS];
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) {
+    const int i = threadIdx.x + s * 256;
+    if (i < nv) gain[s] = reinterpret_cast<const bf16x8*>(w)[i];
+  }
+  pdl_wait();
+  for (int row = blockIdx.x; row < T; row += gridDim.x) {
+    const size_t at = static_cast<size_t>(row) * nv;
+    const bf16x8* xr = reinterpret_cast<const bf16x8*>(x) + at;
+    bf16x8 v[SLOTS], r[SLOTS];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      const int i = threadIdx.x + s * 256;
+      if (i < nv) {
+        v[s] = xr[i];
+        if (res) r[s] = reinterpret_cast<const bf16x8*>(res)[at + i];
+      }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      const int i = threadIdx.x + s * 256;
+      if (i < nv) {
+        float f[8];
+        unpack8(v[s], f);
+        if (res) {
+          float g[8];
+          unpack8(r[s], g);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] += g[j];
+          v[s] = pack8(f);
+          if (res_out) reinterpret_cast<bf16x8*>(res_out)[at + i] = v[s];
+          unpack8(v[s], f);  // normalise what the residual stream actually stores
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+      }
+    }
+    ss = block_sum(ss, red);
+    const float rstd = rsqrtf(ss / H + eps);
+    if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      const int i = threadIdx.x + s * 256;
+      if (i < nv) {
+        float f[8], g[8];
+        unpack8(v[s], f);
+        unpack8(gain[s], g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * g[j];
+        reinterpret_cast<bf16x8*>(y)[at + i] = pack8(f);
+      }
+    }
+  }
+}
+
+// Rows beyond 8192 values do not fit the registers: two passes over memory.
+__global__ void __launch_bounds__(256) rmsnorm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x,
+                                                               const __nv_bfloat16* __restrict__ res,
+                                                               const __nv_bfloat16* __restrict__ w,
+                                                               __nv_bfloat16* __restrict__ y,
+                                                               __nv_bfloat16* __restrict__ res_out,
+                                                               float* __restrict__ rstd_out, int T, int H, float eps) {
+  __shared__ float red[32];
+  pdl_launch_dependents();
   pdl_wait();
   const int nv = H >> 3;
+  auto value = [&](size_t at, float (&f)[8]) {
+    unpack8(reinterpret_cast<const bf16x8*>(x)[at], f);
+    if (res) {
+      float g[8];
+      unpack8(reinterpret_cast<const bf16x8*>(res)[at], g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] += g[j];
+      unpack8(pack8(f), f);  // what the residual stream stores
+    }
+  };
   for (int row = blockIdx.x; row < T; row += gridDim.x) {
-    const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + static_cast<size_t>(row) * H);
-    const bf16x8* rr = res ? reinterpret_cast<const bf16x8*>(res + static_cast<size_t>(row) * H) : nullptr;
-    bf16x8* ro = res_out ? reinterpret_cast<bf16x8*>(res_out + static_cast<size_t>(row) * H) : nullptr;
+    const size_t at = static_cast<size_t>(row) * nv;
     float ss = 0.f;
     for (int i = threadIdx.x; i < nv; i += blockDim.x) {
       float f[8];
-      unpack8(xr[i], f);
-      if (rr) {
-        float g[8];
-        unpack8(rr[i], g);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] += g[j];
-        const bf16x8 s = pack8(f);
-        if (ro) ro[i] = s;
-        unpack8(s, f);  // normalise what the residual stream actually stores
-      }
+      value(at + i, f);
 #pragma unroll
       for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
     }
     ss = block_sum(ss, red);
     const float rstd = rsqrtf(ss / H + eps);
     if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
-    const bf16x8* src = (rr && ro) ? reinterpret_cast<const bf16x8*>(ro) : xr;
-    bf16x8* yr = reinterpret_cast<bf16x8*>(y + static_cast<size_t>(row) * H);
-    const bf16x8* wv = reinterpret_cast<const bf16x8*>(w);
     for (int i = threadIdx.x; i < nv; i += blockDim.x) {
       float f[8], g[8];
-      if (rr && !ro) {
-        float a[8], b[8];
-        unpack8(xr[i], a);
-        unpack8(rr[i], b);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] += b[j];
-        unpack8(pack8(a), f);
-      } else {
-        unpack8(src[i], f);
-      }
-      unpack8(wv[i], g);
+      value(at + i, f);
+      if (res && res_out) reinterpret_cast<bf16x8*>(res_out)[at + i] = pack8(f);
+      unpack8(reinterpret_cast<const bf16x8*>(w)[i], g);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * g[j];
-      yr[i] = pack8(f);
+      reinterpret_cast<bf16x8*>(y)[at + i] = pack8(f);
     }
   }
 }
 
-// dx = rstd * (g*w - x * rstd^2 * mean(g*w*x)) [+ dres] ; partial dw per CTA (reduced by a second kernel).
-constexpr int RMS_SLOTS = 4;  // H <= 256 * 8 * 4 = 8192
+// Rows of at most 256 values (heads): LANES lanes of a warp per row, a CTA of eight warps for 256 / LANES rows.  With a CTA
+// per row 16 of 256 threads had work.
+template <int LANES>
+__global__ void __launch_bounds__(256) rmsnorm_fwd_small_kernel(const __nv_bfloat16* __restrict__ x,
+                                                                const __nv_bfloat16* __restrict__ res,
+                                                                const __nv_bfloat16* __restrict__ w,
+                                                                __nv_bfloat16* __restrict__ y,
+                                                                __nv_bfloat16* __restrict__ res_out,
+                                                                float* __restrict__ rstd_out, int T, int H, float eps) {
+  pdl_launch_dependents();
+  const int nv = H >> 3, i = threadIdx.x % LANES;
+  float g[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (i < nv) unpack8(reinterpret_cast<const bf16x8*>(w)[i], g);
+  pdl_wait();
+  constexpr int ROWS = 256 / LANES;
+  for (long long r0 = static_cast<long long>(blockIdx.x) * ROWS; r0 < T; r0 += static_cast<long long>(gridDim.x) * ROWS) {
+    const long long row = r0 + threadIdx.x / LANES;
+    const bool mine = row < T && i < nv;
+    const size_t at = static_cast<size_t>(row) * nv + i;
+    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, ss = 0.f;
+    if (mine) {
+      unpack8(reinterpret_cast<const bf16x8*>(x)[at], f);
+      if (res) {
+        float a[8];
+        unpack8(reinterpret_cast<const bf16x8*>(res)[at], a);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] += a[j];
+        const bf16x8 sum = pack8(f);
+        if (res_out) reinterpret_cast<bf16x8*>(res_out)[at] = sum;
+        unpack8(sum, f);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    }
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float rstd = rsqrtf(ss / H + eps);
+    if (mine) {
+      if (i == 0 && rstd_out) rstd_out[row] = rstd;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * g[j];
+      reinterpret_cast<bf16x8*>(y)[at] = pack8(f);
+    }
+  }
+}
+
+// dx = rstd * (g*w - x * rstd^2 * mean(g*w*x)) [+ dres] ; partial dw per CTA (reduced by a second kernel).  The gains and a
+// row stay in registers; the next row's loads are under way while the CTA adds up this one's.
+template <int SLOTS>
 __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ g,
                                                           const __nv_bfloat16* __restrict__ x,
                                                           const __nv_bfloat16* __restrict__ w,
@@ -118,49 +227,68 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* _
                                                           float* __restrict__ dw_partial, int T, int H) {
   __shared__ float red[32];
   const int nv = H >> 3;
-  float dw[RMS_SLOTS][8];
+  float dw[SLOTS][8];
+  bf16x8 wv[SLOTS], gv[SLOTS], xv[SLOTS], dv[SLOTS];
 #pragma unroll
-  for (int s = 0; s < RMS_SLOTS; ++s)
+  for (int s = 0; s < SLOTS; ++s) {
+    const int i = threadIdx.x + s * 256;
+    if (i < nv) wv[s] = reinterpret_cast<const bf16x8*>(w)[i];
 #pragma unroll
     for (int j = 0; j < 8; ++j) dw[s][j] = 0.f;
-  const bf16x8* wv = reinterpret_cast<const bf16x8*>(w);
-  for (int row = blockIdx.x; row < T; row += gridDim.x) {
-    const bf16x8* gr = reinterpret_cast<const bf16x8*>(g + static_cast<size_t>(row) * H);
-    const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + static_cast<size_t>(row) * H);
-    const float rs = rstd[row];
-    float dot = 0.f;
+  }
+  float rs = 0.f;
+  auto load = [&](int row) {
+    if (row >= T) return;
+    const size_t at = static_cast<size_t>(row) * nv;
+    rs = rstd[row];
 #pragma unroll
-    for (int s = 0; s < RMS_SLOTS; ++s) {
+    for (int s = 0; s < SLOTS; ++s) {
       const int i = threadIdx.x + s * 256;
       if (i < nv) {
+        gv[s] = reinterpret_cast<const bf16x8*>(g)[at + i];
+        xv[s] = reinterpret_cast<const bf16x8*>(x)[at + i];
+        if (dres) dv[s] = reinterpret_cast<const bf16x8*>(dres)[at + i];
+      }
+    }
+  };
+  load(blockIdx.x);
+  for (int row = blockIdx.x; row < T; row += gridDim.x) {
+    bf16x8 cg[SLOTS], cx[SLOTS], cd[SLOTS];
+    const float crs = rs;
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) { cg[s] = gv[s]; cx[s] = xv[s]; cd[s] = dv[s]; }
+    load(row + gridDim.x);
+    float dot = 0.f;
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      if (threadIdx.x + s * 256 < nv) {
         float gf[8], xf[8], wf[8];
-        unpack8(gr[i], gf);
-        unpack8(xr[i], xf);
-        unpack8(wv[i], wf);
+        unpack8(cg[s], gf);
+        unpack8(cx[s], xf);
+        unpack8(wv[s], wf);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           dot += gf[j] * wf[j] * xf[j];
-          dw[s][j] += gf[j] * xf[j] * rs;
+          dw[s][j] += gf[j] * xf[j] * crs;
         }
       }
     }
     dot = block_sum(dot, red);
-    const float c = dot * rs * rs / H;
-    bf16x8* dxr = reinterpret_cast<bf16x8*>(dx + static_cast<size_t>(row) * H);
-    const bf16x8* dr = dres ? reinterpret_cast<const bf16x8*>(dres + static_cast<size_t>(row) * H) : nullptr;
+    const float c = dot * crs * crs / H;
+    bf16x8* dxr = reinterpret_cast<bf16x8*>(dx) + static_cast<size_t>(row) * nv;
 #pragma unroll
-    for (int s = 0; s < RMS_SLOTS; ++s) {
+    for (int s = 0; s < SLOTS; ++s) {
       const int i = threadIdx.x + s * 256;
       if (i < nv) {
         float gf[8], xf[8], wf[8], o[8];
-        unpack8(gr[i], gf);
-        unpack8(xr[i], xf);
-        unpack8(wv[i], wf);
+        unpack8(cg[s], gf);
+        unpack8(cx[s], xf);
+        unpack8(wv[s], wf);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rs * (gf[j] * wf[j] - xf[j] * c);
-        if (dr) {
+        for (int j = 0; j < 8; ++j) o[j] = crs * (gf[j] * wf[j] - xf[j] * c);
+        if (dres) {
           float d[8];
-          unpack8(dr[i], d);
+          unpack8(cd[s], d);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += d[j];
         }
@@ -170,7 +298,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* _
   }
   float* out = dw_partial + static_cast<size_t>(blockIdx.x) * H;
 #pragma unroll
-  for (int s = 0; s < RMS_SLOTS; ++s) {
+  for (int s = 0; s < SLOTS; ++s) {
     const int i = threadIdx.x + s * 256;
     if (i < nv) {
 #pragma unroll
@@ -179,13 +307,112 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* _
   }
 }
 
-__global__ void colsum_partial_kernel(const float* __restrict__ partial, float* __restrict__ out, int nparts, int H,
-                                      int accumulate) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= H) return;
+// Rows of at most 256 values: LANES lanes per row, two rows of a group under way.
+template <int LANES>
+__global__ void __launch_bounds__(256) rmsnorm_bwd_small_kernel(const __nv_bfloat16* __restrict__ g,
+                                                                const __nv_bfloat16* __restrict__ x,
+                                                                const __nv_bfloat16* __restrict__ w,
+                                                                const float* __restrict__ rstd,
+                                                                const __nv_bfloat16* __restrict__ dres,
+                                                                __nv_bfloat16* __restrict__ dx,
+                                                                float* __restrict__ dw_partial, int T, int H) {
+  constexpr int ROWS = 256 / LANES, U = 2;
+  __shared__ float s_dw[ROWS][LANES * 8];
+  const int nv = H >> 3, i = threadIdx.x % LANES, group = threadIdx.x / LANES;
+  float wf[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, dw[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (i < nv) unpack8(reinterpret_cast<const bf16x8*>(w)[i], wf);
+  const long long step = static_cast<long long>(gridDim.x) * ROWS;
+  for (long long r0 = static_cast<long long>(blockIdx.x) * ROWS; r0 < T; r0 += U * step) {
+    bf16x8 gv[U], xv[U], dv[U];
+    float rs[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long row = r0 + u * step + group;
+      if (row < T && i < nv) {
+        const size_t at = static_cast<size_t>(row) * nv + i;
+        gv[u] = reinterpret_cast<const bf16x8*>(g)[at];
+        xv[u] = reinterpret_cast<const bf16x8*>(x)[at];
+        if (dres) dv[u] = reinterpret_cast<const bf16x8*>(dres)[at];
+        rs[u] = rstd[row];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long row = r0 + u * step + group;
+      const bool mine = row < T && i < nv;
+      float gf[8], xf[8], dot = 0.f;
+      if (mine) {
+        unpack8(gv[u], gf);
+        unpack8(xv[u], xf);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          dot += gf[j] * wf[j] * xf[j];
+          dw[j] += gf[j] * xf[j] * rs[u];
+        }
+      }
+#pragma unroll
+      for (int o = LANES / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+      if (mine) {
+        const float c = dot * rs[u] * rs[u] / H;
+        float o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = rs[u] * (gf[j] * wf[j] - xf[j] * c);
+        if (dres) {
+          float d[8];
+          unpack8(dv[u], d);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] += d[j];
+        }
+        reinterpret_cast<bf16x8*>(dx)[static_cast<size_t>(row) * nv + i] = pack8(o);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) s_dw[group][i * 8 + j] = dw[j];
+  __syncthreads();
+  if (static_cast<int>(threadIdx.x) < H) {
+    float sum = 0.f;
+    for (int k = 0; k < ROWS; ++k) sum += s_dw[k][threadIdx.x];
+    dw_partial[static_cast<size_t>(blockIdx.x) * H + threadIdx.x] = sum;
+  }
+}
+
+// Column sums of the CTAs' partials: 32 columns a CTA, eight threads share a column.
+__global__ void __launch_bounds__(256) colsum_partial_kernel(const float* __restrict__ partial, float* __restrict__ out,
+                                                             int nparts, int H, int accumulate) {
+  __shared__ float s_sum[8][33];
+  const int c = threadIdx.x & 31, k = threadIdx.x >> 5, i = blockIdx.x * 32 + c;
   float s = 0.f;
-  for (int p = 0; p < nparts; ++p) s += partial[static_cast<size_t>(p) * H + i];
-  out[i] = accumulate ? out[i] + s : s;
+  if (i < H) {
+#pragma unroll 8
+    for (int p = k; p < nparts; p += 8) s += partial[static_cast<size_t>(p) * H + i];
+  }
+  s_sum[k][c] = s;
+  __syncthreads();
+  if (k == 0 && i < H) {
+    for (int q = 1; q < 8; ++q) s += s_sum[q][c];
+    out[i] = accumulate ? out[i] + s : s;
+  }
+}
+
+constexpr int RMS_SMALL_H = 256, RMS_MAX_BWD_H = 256 * 8 * 4;
+
+inline int rmsnorm_bwd_launch(const void* g, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
+                              float* dw_partial, float* dw, int dw_accumulate, int T, int H, int parts, cudaStream_t st) {
+  const auto* gp = static_cast<const __nv_bfloat16*>(g);
+  const auto* xp = static_cast<const __nv_bfloat16*>(x);
+  const auto* wp = static_cast<const __nv_bfloat16*>(w);
+  const auto* dp = static_cast<const __nv_bfloat16*>(dres);
+  auto* op = static_cast<__nv_bfloat16*>(dx);
+  auto go = [&](auto kernel) { kernel<<<parts, 256, 0, st>>>(gp, xp, wp, rstd, dp, op, dw_partial, T, H); };
+  if (H <= 64) go(rmsnorm_bwd_small_kernel<8>);
+  else if (H <= 128) go(rmsnorm_bwd_small_kernel<16>);
+  else if (H <= RMS_SMALL_H) go(rmsnorm_bwd_small_kernel<32>);
+  else if (H <= 2048) go(rmsnorm_bwd_kernel<1>);
+  else if (H <= 4096) go(rmsnorm_bwd_kernel<2>);
+  else go(rmsnorm_bwd_kernel<4>);
+  colsum_partial_kernel<<<(H + 31) / 32, 256, 0, st>>>(dw_partial, dw, parts, H, dw_accumulate);
+  return launch_status();
 }
 
 // ------------------------------------------------------------------------------------------ RoPE
@@ -446,12 +673,22 @@ using namespace gk;
 GK_EXPORT int gk_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* res_out, float* rstd,
                              int T, int H, float eps, void* stream) {
   if (H % 8) return -1;
-  const int grid = T < sm_count() * 8 ? T : sm_count() * 8;
-  launch_k(rmsnorm_fwd_kernel, dim3(grid > 0 ? grid : 1), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
-      reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(res),
-      reinterpret_cast<const __nv_bfloat16*>(w), reinterpret_cast<__nv_bfloat16*>(y),
-      reinterpret_cast<__nv_bfloat16*>(res_out), rstd, T, H, eps);
-  return launch_status();
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  auto go = [&](auto kernel, int grid, int threads) {
+    launch_k(kernel, dim3(grid > 0 ? grid : 1), dim3(threads), 0, st, static_cast<const __nv_bfloat16*>(x),
+             static_cast<const __nv_bfloat16*>(res), static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y),
+             static_cast<__nv_bfloat16*>(res_out), rstd, T, H, eps);
+    return launch_status();
+  };
+  const int nv = H / 8, sms = sm_count();
+  if (H <= 64) return go(rmsnorm_fwd_small_kernel<8>, grid_for(T, 32), 256);
+  if (H <= 128) return go(rmsnorm_fwd_small_kernel<16>, grid_for(T, 16), 256);
+  if (H <= RMS_SMALL_H) return go(rmsnorm_fwd_small_kernel<32>, grid_for(T, 8), 256);
+  const int grid = T < sms * 8 ? T : sms * 8;
+  if (nv <= 256) return go(rmsnorm_fwd_kernel<1>, grid, 256);
+  if (nv <= 512) return go(rmsnorm_fwd_kernel<2>, grid, 256);
+  if (nv <= 1024) return go(rmsnorm_fwd_kernel<4>, grid, 256);
+  return go(rmsnorm_fwd_wide_kernel, grid, 256);
 }
 
 // Per-head RMSNorm of the query and key heads of packed [q | k | v] rows, in place (decode / prefill of models with
@@ -511,15 +748,9 @@ GK_EXPORT int gk_rmsnorm_bwd_parts(int T) {
 // dw_partial must hold gk_rmsnorm_bwd_parts(T) * H floats.
 GK_EXPORT int gk_rmsnorm_bwd(const void* g, const void* x, const void* w, const float* rstd, const void* dres,
                              void* dx, float* dw_partial, float* dw, int dw_accumulate, int T, int H, void* stream) {
-  if (H % 8 || H > 256 * 8 * RMS_SLOTS) return -1;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int parts = gk_rmsnorm_bwd_parts(T);
-  rmsnorm_bwd_kernel<<<parts, 256, 0, st>>>(
-      reinterpret_cast<const __nv_bfloat16*>(g), reinterpret_cast<const __nv_bfloat16*>(x),
-      reinterpret_cast<const __nv_bfloat16*>(w), rstd, reinterpret_cast<const __nv_bfloat16*>(dres),
-      reinterpret_cast<__nv_bfloat16*>(dx), dw_partial, T, H);
-  colsum_partial_kernel<<<(H + 255) / 256, 256, 0, st>>>(dw_partial, dw, parts, H, dw_accumulate);
-  return launch_status();
+  if (H % 8 || H > RMS_MAX_BWD_H) return -1;
+  return rmsnorm_bwd_launch(g, x, w, rstd, dres, dx, dw_partial, dw, dw_accumulate, T, H, gk_rmsnorm_bwd_parts(T),
+                            reinterpret_cast<cudaStream_t>(stream));
 }
 
 GK_EXPORT int gk_rope(void* x, const int* pos, int T, int nheads, int D, int rot, long long stride_t, float theta,
@@ -659,11 +890,6 @@ GK_EXPORT int gk_rmsnorm_bwd_noalloc(const void* g, const void* x, const void* w
   float* scratch = g_noalloc_rms_ptr[dev];
   int parts = gk_rmsnorm_bwd_parts(T);
   if (parts > GK_NOALLOC_RMSNORM_MAX_PARTS) parts = GK_NOALLOC_RMSNORM_MAX_PARTS;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  rmsnorm_bwd_kernel<<<parts, 256, 0, st>>>(
-      reinterpret_cast<const __nv_bfloat16*>(g), reinterpret_cast<const __nv_bfloat16*>(x),
-      reinterpret_cast<const __nv_bfloat16*>(w), rstd, reinterpret_cast<const __nv_bfloat16*>(dres),
-      reinterpret_cast<__nv_bfloat16*>(dx), scratch, T, H);
-  colsum_partial_kernel<<<(H + 255) / 256, 256, 0, st>>>(scratch, dw, parts, H, dw_accumulate);
-  return launch_status();
+  return rmsnorm_bwd_launch(g, x, w, rstd, dres, dx, scratch, dw, dw_accumulate, T, H, parts,
+                            reinterpret_cast<cudaStream_t>(stream));
 }
