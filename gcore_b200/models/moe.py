@@ -201,7 +201,7 @@ class _GroupedFp8LinearFn(torch.autograd.Function):
             if fp8_dgrad_enabled() and dy.shape[0] % 128 == 0:
                 dx = quant.fp8_dgrad(dy, ctx.cache, dy.dtype, offsets=offsets, groups=G)
             else:
-                w_dq = quant.dequant_128x128(ctx.cache["q"], ctx.cache["s"])[:G * N, :K].to(dy.dtype).view(G, N, K)
+                w_dq = quant.dequant_128x128_as(ctx.cache["q"], ctx.cache["s"], dy.dtype)[:G * N, :K].view(G, N, K)
                 dx = grouped_gemm(dy, w_dq.contiguous(), offsets, b_mn=True)
         if ctx.needs_input_grad[1]:
             if ctx.main_grad is not None:

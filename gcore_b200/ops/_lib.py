@@ -205,6 +205,11 @@ def _declare_kernels(lib: ctypes.CDLL):
     d("gk_sample", [P, I, L, I, I, F, I, P, P, P, P, P, I, I, P])
     d("gk_sample_combine", [P, I, I, P, P, P])
     d("gk_sample_filtered", [P, I, L, I, F, I, F, F, I, P, P, P, P, P, I, P])
+    d("gk_rope_copy", [P, P, P, I, I, I, I, I, F, I, I, P])
+    d("gk_dequant_128x128", [P, P, P, L, I, P])
+    d("gk_mla_expand", [P, P, P, P, I, I, I, I, I, P])
+    d("gk_mla_expand_bwd", [P, P, P, P, I, I, I, I, I, P])
+    d("gk_latent_append", [P, L, P, P, P, P, I, I, I, F, F, I, P])
     d("gk_decode_begin", [P, P, P])
     d("gk_decode_end", [P, I, I, P])
     d("gk_grpo_loss", [P, P, P, P, P, L, F, F, F, F, F, F, P, P, P, P])

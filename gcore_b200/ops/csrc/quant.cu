@@ -146,6 +146,29 @@ __global__ void fp4_quant_1x32_kernel(const __nv_bfloat16* __restrict__ x, uint8
   }
 }
 
+// bf16 values of e4m3 codes [rows, K] with one scale per 128 x 128 block, 16 codes per thread: three bytes of traffic a value.
+// 36864 x 7168: 140 us (floor 123), 1959 as tensor operations through fp32.
+__global__ void __launch_bounds__(256) dequant_128x128_kernel(const uint4* __restrict__ q, const float* __restrict__ s,
+                                                              uint4* __restrict__ out, long long units, int per_row, int kb) {
+  for (long long u = blockIdx.x * 256ll + threadIdx.x; u < units; u += gridDim.x * 256ll) {
+    const long long row = u / per_row;
+    const int c = static_cast<int>(u - row * per_row);
+    const float sc = s[(row >> 7) * kb + (c >> 3)];
+    const uint4 r = __ldcs(q + u);
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+    uint32_t o[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const __nv_fp8x2_storage_t two = static_cast<__nv_fp8x2_storage_t>(w[i >> 1] >> (16 * (i & 1)));
+      const __half2 h = __half2(__nv_cvt_fp8x2_to_halfraw2(two, __NV_E4M3));
+      const __nv_bfloat162 b = __floats2bfloat162_rn(__low2float(h) * sc, __high2float(h) * sc);
+      o[i] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+    out[2 * u] = make_uint4(o[0], o[1], o[2], o[3]);
+    out[2 * u + 1] = make_uint4(o[4], o[5], o[6], o[7]);
+  }
+}
+
 }  // namespace gq
 
 using namespace gq;
@@ -180,5 +203,16 @@ GK_EXPORT int gk_fp4_quant_1x32(const void* x, void* packed, void* scale_e8m0, f
   fp4_quant_1x32_kernel<<<static_cast<unsigned>((nb + 127) / 128), 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<uint8_t*>(packed),
       reinterpret_cast<uint8_t*>(scale_e8m0), scale_f32, reinterpret_cast<__nv_bfloat16*>(dq), nb);
+  return gk::launch_status();
+}
+
+// q [N, K] e4m3 (K a multiple of 128, 16-byte aligned), s [ceil(N / 128), K / 128] -> out [N, K] bf16.
+GK_EXPORT int gk_dequant_128x128(const void* q, const float* s, void* out, long long N, int K, void* stream) {
+  if (K % 128 || ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15)) return -1;
+  const long long units = N * (K / 16);
+  if (units == 0) return 0;
+  const long long want = (units + 255) / 256, most = gk::sm_count() * 32ll;
+  gq::dequant_128x128_kernel<<<static_cast<unsigned>(want < most ? want : most), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      static_cast<const uint4*>(q), s, static_cast<uint4*>(out), units, K / 16, K / 128);
   return gk::launch_status();
 }

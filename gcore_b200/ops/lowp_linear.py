@@ -102,7 +102,7 @@ class _Fp8LinearFn(torch.autograd.Function):
             if fp8_dgrad_enabled() and w.shape[0] % 128 == 0 and w.shape[1] % 128 == 0:
                 dx = quant.fp8_dgrad(dy2, ctx.cache, dy2.dtype)
             else:
-                w_dq = quant.dequant_128x128(ctx.cache["q"], ctx.cache["s"]).to(dy2.dtype)
+                w_dq = quant.dequant_128x128_as(ctx.cache["q"], ctx.cache["s"], dy2.dtype)
                 dx = linear_dgrad(dy2, w_dq[:w.shape[0], :w.shape[1]].contiguous())
         if ctx.needs_input_grad[1]:
             if fp8_wgrad_enabled() and w.shape[0] % 128 == 0 and w.shape[1] % 128 == 0:

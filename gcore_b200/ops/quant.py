@@ -54,6 +54,20 @@ def dequant_128x128(q: torch.Tensor, s: torch.Tensor) -> torch.Tensor:
     return q.float() * s.repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)[:, :K]
 
 
+def dequant_128x128_as(q: torch.Tensor, s: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """``dequant_128x128(q, s).to(dtype)``, in one pass for bf16 on a GPU."""
+    N, K = q.shape
+    if (dtype == torch.bfloat16 and _lib.use_native(q) and K % 128 == 0 and q.dtype == torch.float8_e4m3fn and q.is_contiguous()
+            and s.dtype == torch.float32 and s.is_contiguous() and tuple(s.shape) == ((N + 127) // 128, K // 128)
+            and q.data_ptr() % 16 == 0 and N > 0):
+        out = torch.empty(N, K, dtype=dtype, device=q.device)
+        LAUNCHES["quant"] += 1
+        _lib.check(_lib.kernels().gk_dequant_128x128(_lib.ptr(q), _lib.ptr(s), _lib.ptr(out), N, K, _lib.stream_ptr()),
+                   "dequant_128x128")
+        return out
+    return dequant_128x128(q, s).to(dtype)
+
+
 def fp4_quant_1x32_ref(x: torch.Tensor):
     """Returns (codes uint8 [numel] with sign in bit 3, scale fp32 [numel/32], dequantised fp32)."""
     xf = x.float().reshape(-1, 32)
