@@ -23,7 +23,7 @@ import torch.nn as nn
 from torch.utils.checkpoint import checkpoint
 
 from ..core import parallel_state as ps
-from ..ops import fused
+from ..ops import _lib, fused
 from ..ops.attention import flash_attn_qkvpacked, flash_attn_varlen
 from ..ops.gemm import linear
 from ..parallel import tp_ops
@@ -220,24 +220,63 @@ class MLAttention(nn.Module):
         self.linear_proj = ParallelLinear(cfg.num_attention_heads * dv, H, "row", cfg, tp_size=tp_size,
                                           init_std=cfg.init_std / math.sqrt(2 * cfg.num_layers), device=device)
 
+    def _query(self, x):
+        """``[T, heads, dn + dr]``, the last ``dr`` values of a head not yet rotated."""
+        if self.cfg.q_lora_rank:
+            ql = fused.rmsnorm(self.linear_q_down_proj(x), self.q_layernorm.weight, self.cfg.rms_norm_eps)[0]
+            return self.linear_q_up_proj(ql).view(x.shape[0], self.h, self.cfg.qk_head_dim)
+        return self.linear_q_proj(x).view(x.shape[0], self.h, self.cfg.qk_head_dim)
+
+    def _latent(self, x, pos):
+        """The normalised latent ``c_kv [T, kv_lora]`` and the rotated shared key ``k_rope [T, dr]``."""
+        cfg = self.cfg
+        T, dr = x.shape[0], cfg.qk_rope_head_dim
+        kv = self.linear_kv_down_proj(x)
+        c_kv, k_rope = kv.split([cfg.kv_lora_rank, dr], dim=-1)
+        c_kv = fused.rmsnorm(c_kv.contiguous(), self.kv_layernorm.weight, cfg.rms_norm_eps)[0]
+        k_rope = fused.rope(k_rope.reshape(T, 1, dr).contiguous(), pos, cfg.rope_theta, dr, cfg.rope_interleaved)
+        return c_kv, k_rope.reshape(T, dr)
+
+    def _rotates_whole(self, x, pos) -> bool:
+        """Whether the query's rotated part is turned where it lies (bf16 on a GPU, plain positions, whole 16-byte units)."""
+        cfg = self.cfg
+        return (_lib.use_native(x) and x.dtype == torch.bfloat16 and isinstance(pos, torch.Tensor) and pos.dim() == 1
+                and cfg.qk_nope_head_dim % 8 == 0 and cfg.qk_rope_head_dim % 16 == 0 and cfg.qk_rope_head_dim <= 512)
+
+    def _rotated_query(self, x, pos):
+        cfg = self.cfg
+        q = self._query(x)
+        q = q if q.is_contiguous() and q.data_ptr() % 16 == 0 else q.clone(memory_format=torch.contiguous_format)
+        return fused.RotateTail.apply(q, pos.to(torch.int32).contiguous(), cfg.rope_theta, cfg.qk_rope_head_dim,
+                                      cfg.rope_interleaved)
+
     def project(self, x, pos):
         """Per-token projections: ``q_nope [T, h, dn]``, rotated ``q_rope [T, h, dr]``, the normalised latent
         ``c_kv [T, kv_lora]`` and the rotated shared key ``k_rope [T, dr]`` (the last two are what a decoder caches)."""
         cfg = self.cfg
-        T, h = x.shape[0], self.h
-        dn, dr = cfg.qk_nope_head_dim, cfg.qk_rope_head_dim
-        if cfg.q_lora_rank:
-            ql = fused.rmsnorm(self.linear_q_down_proj(x), self.q_layernorm.weight, cfg.rms_norm_eps)[0]
-            q = self.linear_q_up_proj(ql).view(T, h, dn + dr)
-        else:
-            q = self.linear_q_proj(x).view(T, h, dn + dr)
-        kv = self.linear_kv_down_proj(x)
-        c_kv, k_rope = kv.split([cfg.kv_lora_rank, dr], dim=-1)
-        c_kv = fused.rmsnorm(c_kv.contiguous(), self.kv_layernorm.weight, cfg.rms_norm_eps)[0]
-        q_nope, q_rope = q.split([dn, dr], dim=-1)
-        q_rope = fused.rope(q_rope.contiguous(), pos, cfg.rope_theta, dr, cfg.rope_interleaved)
-        k_rope = fused.rope(k_rope.reshape(T, 1, dr).contiguous(), pos, cfg.rope_theta, dr, cfg.rope_interleaved)
-        return q_nope, q_rope, c_kv, k_rope.reshape(T, dr)
+        q_nope, q_rope = self._query(x).split([cfg.qk_nope_head_dim, cfg.qk_rope_head_dim], dim=-1)
+        q_rope = fused.rope(q_rope.contiguous(), pos, cfg.rope_theta, cfg.qk_rope_head_dim, cfg.rope_interleaved)
+        return q_nope, q_rope, *self._latent(x, pos)
+
+    def packed_ready(self, x, pos, cu_seqlens) -> bool:
+        """Whether ``attend_packed`` serves the batch: the wide-key flash kernels on whole sequences of one rank."""
+        cfg = self.cfg
+        return (self._rotates_whole(x, pos) and not isinstance(cu_seqlens, CPContext) and cfg.qk_rope_head_dim in (16, 32, 64, 128, 256)
+                and (cfg.qk_head_dim, cfg.v_head_dim) == (192, 128) and os.environ.get("GCORE_MLA_FLASH", "1") != "0")
+
+    def attend_packed(self, q, c_kv, k_rope, cu_seqlens, max_seqlen=None):
+        """``attend`` for the rotated query [T, h, dn + dr]: keys and values leave the up-projection in one pass."""
+        from ..ops.attention import flash_attn_varlen
+        cfg = self.cfg
+        T, dn, dv = q.shape[0], cfg.qk_nope_head_dim, cfg.v_head_dim
+        kvu = self.linear_kv_up_proj(c_kv).view(T, self.h, dn + dv)
+        kvu = kvu if kvu.is_contiguous() and kvu.data_ptr() % 16 == 0 else kvu.clone(memory_format=torch.contiguous_format)
+        k, v = fused.ExpandLatent.apply(kvu, k_rope.contiguous(), dn)
+        if max_seqlen is None:
+            max_seqlen = int((cu_seqlens[1:] - cu_seqlens[:-1]).max())
+        o = flash_attn_varlen(q, k, v, cu_seqlens, cu_seqlens, max_seqlen, max_seqlen, causal=True,
+                              scale=1.0 / math.sqrt(cfg.qk_head_dim))
+        return o.reshape(T, self.h * dv)
 
     def attend(self, q_nope, q_rope, c_kv, k_rope, cu_seqlens, max_seqlen=None):
         """Causal attention over packed sequences with the latent expanded to per-head keys and values."""
@@ -296,6 +335,8 @@ class MLAttention(nn.Module):
         return o[..., :dv].reshape(T, h * dv)
 
     def forward(self, x, pos, cu_seqlens, max_seqlen):
+        if self.packed_ready(x, pos, cu_seqlens):
+            return self.linear_proj(self.attend_packed(self._rotated_query(x, pos), *self._latent(x, pos), cu_seqlens, max_seqlen))
         return self.linear_proj(self.attend(*self.project(x, pos), cu_seqlens, max_seqlen))
 
 

@@ -442,6 +442,63 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict
   }
 }
 
+// The same for aligned rows: 16-byte units, and one angle for all heads of a token, ROPE_TOKENS tokens a CTA.  Rotates the
+// values [off, off + rot) of every head; with y != x the other values are copied.  8000 tokens of 32 heads of 128: 41 us against
+// 84 a pair at a time, 26000 tokens of 40 heads 139 against 309.
+constexpr int ROPE_TOKENS = 4, ROPE_MAX_ROT = 512;
+__global__ void __launch_bounds__(256) rope_rows_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const int* __restrict__ pos,
+                                                        int T, int nheads, int D, int off, int rot, long long ldx, long long ldy,
+                                                        float theta, float sign, int interleaved) {
+  __shared__ float2 cs[ROPE_TOKENS * ROPE_MAX_ROT / 2];
+  const int half = rot >> 1, t0 = blockIdx.x * ROPE_TOKENS, n = T - t0 < ROPE_TOKENS ? T - t0 : ROPE_TOKENS;
+  for (int k = threadIdx.x; k < n * half; k += 256) {
+    const int tok = k / half, i = k - tok * half;
+    const float inv = __powf(theta, -2.f * i / rot);
+    float s, c;
+    sincosf(pos[t0 + tok] * inv, &s, &c);
+    cs[k] = make_float2(c, s * sign);
+  }
+  __syncthreads();
+  const unsigned turned = interleaved ? rot >> 3 : rot >> 4;               // units of a head that rotate: one or two vectors
+  const unsigned lead = off >> 3, kept = x == y ? 0 : (D - rot) >> 3;      // vectors that are copied, `lead` of them in front
+  const unsigned per = turned + kept, units = n * nheads * per;
+  for (unsigned u = threadIdx.x; u < units; u += 256) {
+    const unsigned th = u / per, k = u - th * per, tok = th / nheads, h = th - tok * nheads;
+    const bf16x8* from = reinterpret_cast<const bf16x8*>(x + (t0 + tok) * ldx + static_cast<long long>(h) * D);
+    bf16x8* to = reinterpret_cast<bf16x8*>(y + (t0 + tok) * ldy + static_cast<long long>(h) * D);
+    if (k >= turned) {
+      const unsigned c = k - turned < lead ? k - turned : k - turned + (rot >> 3);
+      to[c] = from[c];
+      continue;
+    }
+    const float2* ang = cs + tok * half;
+    if (interleaved) {
+      float f[8];
+      unpack8(from[lead + k], f);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float c = ang[4 * k + j].x, s = ang[4 * k + j].y, a = f[2 * j], b = f[2 * j + 1];
+        f[2 * j] = a * c - b * s;
+        f[2 * j + 1] = b * c + a * s;
+      }
+      to[lead + k] = pack8(f);
+    } else {
+      const unsigned other = lead + k + (half >> 3);
+      float f[8], g[8];
+      unpack8(from[lead + k], f);
+      unpack8(from[other], g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float c = ang[8 * k + j].x, s = ang[8 * k + j].y, a = f[j], b = g[j];
+        f[j] = a * c - b * s;
+        g[j] = b * c + a * s;
+      }
+      to[lead + k] = pack8(f);
+      to[other] = pack8(g);
+    }
+  }
+}
+
 // Same rotation with the angles given as tables cos / sin [T, rot / 2] (multi-axis rotary position ids of
 // vision-language models: every frequency takes its angle from the temporal, height or width index of the token).
 __global__ void rope_table_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cs,
@@ -753,11 +810,34 @@ GK_EXPORT int gk_rmsnorm_bwd(const void* g, const void* x, const void* w, const 
                             reinterpret_cast<cudaStream_t>(stream));
 }
 
+static bool rope_rows_ok(const void* x, const void* y, int D, int off, int rot, long long ldx, long long ldy, int interleaved) {
+  return D % 8 == 0 && off % 8 == 0 && rot % (interleaved ? 8 : 16) == 0 && rot >= 8 && rot <= ROPE_MAX_ROT && off + rot <= D &&
+         ldx % 8 == 0 && ldy % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+}
+
+// y = x [T, nheads, D] (contiguous rows, 16-byte aligned, y != x) with the values [off, off + rot) of every head rotated.
+GK_EXPORT int gk_rope_copy(const void* x, void* y, const int* pos, int T, int nheads, int D, int off, int rot, float theta,
+                           int backward, int interleaved, void* stream) {
+  const long long ld = static_cast<long long>(nheads) * D;
+  if (x == y || !rope_rows_ok(x, y, D, off, rot, ld, ld, interleaved)) return -1;
+  if (T == 0) return 0;
+  rope_rows_kernel<<<(T + ROPE_TOKENS - 1) / ROPE_TOKENS, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), pos, T, nheads, D, off, rot, ld, ld, theta,
+      backward ? -1.f : 1.f, interleaved);
+  return launch_status();
+}
+
 GK_EXPORT int gk_rope(void* x, const int* pos, int T, int nheads, int D, int rot, long long stride_t, float theta,
                       int backward, int interleaved, void* stream) {
   if (rot % 2 || rot > D) return -1;
   const long long total = static_cast<long long>(T) * nheads * (rot / 2);
   if (total == 0) return 0;
+  if (rope_rows_ok(x, x, D, 0, rot, stride_t, stride_t, interleaved)) {
+    rope_rows_kernel<<<(T + ROPE_TOKENS - 1) / ROPE_TOKENS, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(x), pos, T, nheads, D, 0, rot, stride_t, stride_t,
+        theta, backward ? -1.f : 1.f, interleaved);
+    return launch_status();
+  }
   rope_kernel<<<grid_for(total, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<__nv_bfloat16*>(x), pos, T, nheads, D, rot, stride_t, theta, backward ? -1.f : 1.f,
       interleaved);

@@ -165,6 +165,65 @@ def rope(x, pos, theta, rot=None, interleaved=False):
     return _RopeFn.apply(x, pos, theta, rot, interleaved)
 
 
+class RotateTail(torch.autograd.Function):
+    """``x`` [T, heads, D] (bf16 on a GPU, contiguous) with the last ``rot`` values of every head rotated; ``pos`` int32."""
+
+    @staticmethod
+    def forward(ctx, x, pos, theta, rot, interleaved):
+        ctx.save_for_backward(pos)
+        ctx.args = (theta, rot, interleaved)
+        return RotateTail._turn(x, pos, theta, rot, interleaved, 0)
+
+    @staticmethod
+    def backward(ctx, g):
+        (pos,) = ctx.saved_tensors
+        return RotateTail._turn(g.contiguous(), pos, *ctx.args, 1), None, None, None, None
+
+    @staticmethod
+    def _turn(x, pos, theta, rot, interleaved, backward):
+        (T, nh, D), y = x.shape, torch.empty_like(x)
+        LAUNCHES["elementwise"] += 1
+        _lib.check(_lib.kernels().gk_rope_copy(_lib.ptr(x), _lib.ptr(y), _lib.ptr(pos), T, nh, D, D - rot, rot, float(theta),
+                                               backward, int(interleaved), _lib.stream_ptr()), "rope_copy")
+        return y
+
+
+class ExpandLatent(torch.autograd.Function):
+    """Keys ``[T, heads, dn + dr]`` and values ``[T, heads, dv]`` from the up-projected latent ``kvu`` [T, heads, dn + dv] and
+    the shared rotated key ``kr`` [T, dr] (bf16 on a GPU, contiguous)."""
+
+    @staticmethod
+    def forward(ctx, kvu, kr, dn):
+        (T, h, w), dr = kvu.shape, kr.shape[1]
+        k = torch.empty(T, h, dn + dr, dtype=kvu.dtype, device=kvu.device)
+        v = torch.empty(T, h, w - dn, dtype=kvu.dtype, device=kvu.device)
+        ctx.sizes = (T, h, dn, dr, w - dn)
+        LAUNCHES["elementwise"] += 1
+        _lib.check(_lib.kernels().gk_mla_expand(_lib.ptr(kvu), _lib.ptr(kr), _lib.ptr(k), _lib.ptr(v), T, h, dn, dr, w - dn,
+                                                _lib.stream_ptr()), "mla_expand")
+        return k, v
+
+    @staticmethod
+    def backward(ctx, dk, dv):
+        T, h, dn, dr, w = ctx.sizes
+        dk, dv = dk.contiguous(), dv.contiguous()
+        dkvu = torch.empty(T, h, dn + w, dtype=dk.dtype, device=dk.device)
+        dkr = torch.empty(T, dr, dtype=dk.dtype, device=dk.device)
+        LAUNCHES["elementwise"] += 1
+        _lib.check(_lib.kernels().gk_mla_expand_bwd(_lib.ptr(dk), _lib.ptr(dv), _lib.ptr(dkvu), _lib.ptr(dkr), T, h, dn, dr, w,
+                                                    _lib.stream_ptr()), "mla_expand_bwd")
+        return dkvu, dkr, None
+
+
+def latent_append(kv, gain, pos, slots, cache, kv_lora: int, eps: float, theta: float, interleaved: bool):
+    """One decode token per request: RMSNorm of the latent ``kv[:, :kv_lora]`` and the rotation of the shared key behind it,
+    written to the rows ``slots`` (int64) of ``cache`` [rows, kv_lora + dr] (bf16 on a GPU)."""
+    LAUNCHES["elementwise"] += 1
+    _lib.check(_lib.kernels().gk_latent_append(_lib.ptr(kv), kv.stride(0), _lib.ptr(gain), _lib.ptr(pos), _lib.ptr(slots),
+                                               _lib.ptr(cache), kv.shape[0], kv_lora, cache.shape[1] - kv_lora, float(eps),
+                                               float(theta), int(interleaved), _lib.stream_ptr()), "latent_append")
+
+
 # ------------------------------------------------------------------------------------------------ SwiGLU
 def qk_headnorm_(qkv: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor, Hq: int, Hk: int, D: int, eps: float):
     """In-place per-head RMSNorm of the query and key heads of packed ``[T, (Hq + 2 Hk) * D]`` rows (inference: no

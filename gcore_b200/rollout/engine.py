@@ -581,12 +581,17 @@ class InferEngine:
         for li, lw in enumerate(self.w.layers):
             h, res = fused.rmsnorm(x, lw.ln1, cfg.rms_norm_eps, res)
             if lw.mla is not None:
-                q_nope, q_rope, c_kv, k_rope = lw.mla.project(h, pos)
+                packed = lw.mla.packed_ready(h, pos, cu)
+                if packed:
+                    q, (c_kv, k_rope) = lw.mla._rotated_query(h, pos), lw.mla._latent(h, pos)
+                else:
+                    q_nope, q_rope, c_kv, k_rope = lw.mla.project(h, pos)
                 sink = (self.k_cache[li].shape[0] - 1) * self.bs  # rows without a slot land in the spare block
                 self.k_cache[li].view(-1, self.mla_dim).index_copy_(
                     0, torch.where(slots >= 0, slots, torch.full_like(slots, sink)).long(),
                     torch.cat([self._mla_cached_latent(lw.mla, c_kv), k_rope], -1))
-                a = self._allreduce(lw.mla.linear_proj(lw.mla.attend(q_nope, q_rope, c_kv, k_rope, cu, max_len)))
+                a = self._allreduce(lw.mla.linear_proj(lw.mla.attend_packed(q, c_kv, k_rope, cu, max_len) if packed else
+                                                       lw.mla.attend(q_nope, q_rope, c_kv, k_rope, cu, max_len)))
                 h, res = fused.rmsnorm(a, lw.ln2, cfg.rms_norm_eps, res)
                 x = self._mlp(lw, h)
                 continue
@@ -762,6 +767,15 @@ class InferEngine:
         return hasattr(lib, "gk_mla_decode_supported") and \
             bool(lib.gk_mla_decode_supported(cfg.kv_lora_rank, cfg.qk_rope_head_dim))
 
+    def _latent_appends(self, mla, h, pos, flat) -> bool:
+        """Whether a decode step's latents go to the cache in one kernel (bf16, no fp8 image of the latent, whole 16-byte
+        units)."""
+        cfg, gain = self.cfg, mla.kv_layernorm.weight
+        return (mla._rotates_whole(h, pos) and pos.dtype == torch.int32 and flat.dtype == torch.bfloat16
+                and gain.dtype == torch.bfloat16 and gain.data_ptr() % 16 == 0 and flat.data_ptr() % 16 == 0
+                and getattr(mla.linear_kv_up_proj, "precision", None) != "fp8"
+                and cfg.kv_lora_rank % 8 == 0 and cfg.kv_lora_rank <= 1024)
+
     def _mla_decode(self, mla, h, pos, cache, slots, lat_idx, lat_mask, paged=None):
         """One token per request of multi-head latent attention on the latent cache, in the absorbed form: the key
         up-projection is folded into the query and the value up-projection is applied after the weighted sum, so a
@@ -770,9 +784,15 @@ class InferEngine:
         cfg = self.cfg
         dn, dr, dv, C = cfg.qk_nope_head_dim, cfg.qk_rope_head_dim, cfg.v_head_dim, cfg.kv_lora_rank
         B = h.shape[0]
-        q_nope, q_rope, c_kv, k_rope = mla.project(h, pos)
         flat = cache.view(-1, self.mla_dim)
-        flat.index_copy_(0, slots, torch.cat([self._mla_cached_latent(mla, c_kv), k_rope], -1))
+        if self._latent_appends(mla, h, pos, flat):
+            kv = mla.linear_kv_down_proj(h)
+            fused.latent_append(kv, mla.kv_layernorm.weight, pos, slots, flat, C, cfg.rms_norm_eps, cfg.rope_theta,
+                                cfg.rope_interleaved)
+            q_nope, q_rope = mla._rotated_query(h, pos).split([dn, dr], dim=-1)
+        else:
+            q_nope, q_rope, c_kv, k_rope = mla.project(h, pos)
+            flat.index_copy_(0, slots, torch.cat([self._mla_cached_latent(mla, c_kv), k_rope], -1))
         w_up = self._mla_absorbed(mla)
         if lat_idx is None:
             # latent decode kernel straight on the paged cache: the two absorbed projections are head-batched GEMMs
