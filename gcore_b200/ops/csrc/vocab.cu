@@ -136,30 +136,82 @@ __global__ void logprob_entropy_combine_kernel(const float* __restrict__ partial
   if (ent) ent[t] = lse - o.sz / o.s;
 }
 
-// d logit_j = inv_temp * [ g_lp * (1{j==y} - p_j) - g_H * p_j * (z_j - lse + H) ], written over the logits.
-__global__ void __launch_bounds__(256) logprob_entropy_bwd_kernel(void* __restrict__ logits, int is_fp32, long long ld,
+// d logit_j = inv_temp * [ g_lp * (1{j==y} - p_j) - g_H * p_j * (z_j - lse + H) ], written over the logits.  VEC: rows start at
+// 16 bytes, a thread takes 16 bytes at a time (two bytes at a time the pass ran at a quarter of HBM's rate).
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256) logprob_entropy_bwd_kernel(T* __restrict__ logits, long long ld,
                                                                   const long long* __restrict__ targets,
                                                                   const float* __restrict__ lse,
                                                                   const float* __restrict__ ent,
                                                                   const float* __restrict__ g_lp,
                                                                   const float* __restrict__ g_ent, float inv_temp,
                                                                   int vocab_start, int V) {
+  constexpr int W = VEC ? 16 / static_cast<int>(sizeof(T)) : 1;
+  struct alignas(W * sizeof(T)) Pack { T e[W]; };
   const long long row = blockIdx.x;
-  const long long base = row * ld;
+  T* z0 = logits + row * ld;
   const float l = lse[row];
   const float H = ent ? ent[row] : 0.f;
   const float gl = g_lp ? g_lp[row] : 0.f;
   const float gh = g_ent ? g_ent[row] : 0.f;
   const long long tg = targets[row] - vocab_start;
-  for (int j = threadIdx.x; j < V; j += blockDim.x) {
-    const float z = load_logit(logits, is_fp32, base + j) * inv_temp;
+  auto grad = [&](float logit, int j) {
+    const float z = logit * inv_temp;
     const float p = __expf(z - l);
     float d = gl * ((j == tg ? 1.f : 0.f) - p);
     if (g_ent) d -= gh * p * (z - l + H);
-    d *= inv_temp;
-    if (is_fp32) reinterpret_cast<float*>(logits)[base + j] = d;
-    else reinterpret_cast<__nv_bfloat16*>(logits)[base + j] = __float2bfloat16(d);
+    return d * inv_temp;
+  };
+  const int packs = V / W;
+#pragma unroll 2
+  for (int k = threadIdx.x; k < packs; k += 256) {
+    Pack v = reinterpret_cast<const Pack*>(z0)[k];
+#pragma unroll
+    for (int i = 0; i < W; ++i) v.e[i] = static_cast<T>(grad(static_cast<float>(v.e[i]), k * W + i));
+    reinterpret_cast<Pack*>(z0)[k] = v;
   }
+  for (int j = packs * W + threadIdx.x; j < V; j += 256) z0[j] = static_cast<T>(grad(static_cast<float>(z0[j]), j));
+}
+
+// Gradient of an embedding table in fp32, added to what is there: the CTA at the first of a run of equal tokens (sorted, with
+// their rows) adds up the run's rows in order.  Through autograd's own operation the sum was a dense bf16 table, cleared,
+// converted and added to the fp32 one.  With the logits' gradient above, policy updates: dense 31.2 -> 30.2 ms, mixture of
+// experts 11.9 -> 11.1.
+__global__ void __launch_bounds__(256) embedding_grad_kernel(const long long* __restrict__ ids, const long long* __restrict__ rows,
+                                                             const uint4* __restrict__ dy, float4* __restrict__ grad, int n,
+                                                             int vecs, long long V) {
+  const int i = blockIdx.x, c = blockIdx.y * 256 + threadIdx.x;
+  const long long id = ids[i];
+  if ((i > 0 && ids[i - 1] == id) || id < 0 || id >= V || c >= vecs) return;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  constexpr int U = 4;
+  for (int j = i; j < n; j += U) {
+    uint4 v[U];
+    bool same[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      same[u] = j + u < n && ids[j + u] == id;
+      v[u] = dy[rows[same[u] ? j + u : i] * vecs + c];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (!same[u]) break;
+      const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v[u]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 f = __bfloat1622float2(e[k]);
+        acc[2 * k] += f.x;
+        acc[2 * k + 1] += f.y;
+      }
+    }
+    if (!same[U - 1]) break;
+  }
+  float4* g = grad + (id * vecs + c) * 2;
+  float4 a = g[0], b = g[1];
+  a.x += acc[0]; a.y += acc[1]; a.z += acc[2]; a.w += acc[3];
+  b.x += acc[4]; b.y += acc[5]; b.z += acc[6]; b.w += acc[7];
+  g[0] = a;
+  g[1] = b;
 }
 
 // Gumbel-max: argmax_j (z_j + G_j) is a sample from softmax(z).  One CTA per request.
@@ -418,8 +470,27 @@ GK_EXPORT int gk_logprob_entropy_bwd(void* logits, int is_fp32, long long ld, co
                                      const float* lse, const float* ent, const float* g_lp, const float* g_ent,
                                      float inv_temp, int vocab_start, int V, long long T, void* stream) {
   if (T == 0) return 0;
-  logprob_entropy_bwd_kernel<<<static_cast<unsigned>(T), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      logits, is_fp32, ld, targets, lse, ent, g_lp, g_ent, inv_temp, vocab_start, V);
+  const bool vec = (reinterpret_cast<uintptr_t>(logits) & 15) == 0 && ld * (is_fp32 ? 4 : 2) % 16 == 0;
+  auto go = [&](auto* z, auto kernel) {
+    kernel<<<static_cast<unsigned>(T), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(z, ld, targets, lse, ent, g_lp, g_ent,
+                                                                                         inv_temp, vocab_start, V);
+    return launch_status();
+  };
+  if (is_fp32) {
+    auto* z = static_cast<float*>(logits);
+    return vec ? go(z, logprob_entropy_bwd_kernel<float, true>) : go(z, logprob_entropy_bwd_kernel<float, false>);
+  }
+  auto* z = static_cast<__nv_bfloat16*>(logits);
+  return vec ? go(z, logprob_entropy_bwd_kernel<__nv_bfloat16, true>) : go(z, logprob_entropy_bwd_kernel<__nv_bfloat16, false>);
+}
+
+// ids sorted, rows: where in dy [n, H] (bf16) each lies; grad [V, H] fp32.  H a multiple of 8, 16-byte aligned.
+GK_EXPORT int gk_embedding_grad(const long long* ids, const long long* rows, const void* dy, float* grad, int n, int H,
+                                long long V, void* stream) {
+  if (H % 8 || H < 8 || H / 8 > 256 * 65535) return -1;
+  if (n == 0) return 0;
+  embedding_grad_kernel<<<dim3(n, (H / 8 + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      ids, rows, static_cast<const uint4*>(dy), reinterpret_cast<float4*>(grad), n, H / 8, V);
   return launch_status();
 }
 

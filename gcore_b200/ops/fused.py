@@ -77,6 +77,40 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6, residual: torch
     return rmsnorm_ref(x, w, eps, residual)
 
 
+# ------------------------------------------------------------------------------------------------ embedding
+class _EmbeddingFn(torch.autograd.Function):
+    """Embedding rows; the table's gradient is added to its fp32 ``main_grad`` (rows of equal tokens in the order of the
+    batch), autograd sees none."""
+
+    @staticmethod
+    def forward(ctx, ids, weight, main_grad):
+        ctx.save_for_backward(ids)
+        ctx.main_grad = main_grad
+        return torch.nn.functional.embedding(ids, weight)
+
+    @staticmethod
+    def backward(ctx, g):
+        (ids,) = ctx.saved_tensors
+        V, H = ctx.main_grad.shape
+        g = g.reshape(-1, H)
+        g = g if g.is_contiguous() and g.data_ptr() % 16 == 0 else g.clone(memory_format=torch.contiguous_format)
+        order, rows = torch.sort(ids.reshape(-1), stable=True)
+        LAUNCHES["elementwise"] += 1
+        _lib.check(_lib.kernels().gk_embedding_grad(_lib.ptr(order), _lib.ptr(rows), _lib.ptr(g), _lib.ptr(ctx.main_grad),
+                                                    rows.numel(), H, V, _lib.stream_ptr()), "embedding_grad")
+        return None, None, None
+
+
+def embedding(ids: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """``weight[ids]``; a bf16 table with an fp32 ``main_grad`` on a GPU collects its gradient there."""
+    mg = getattr(weight, "main_grad", None) if weight.requires_grad and torch.is_grad_enabled() else None
+    if (mg is not None and _lib.use_native(weight) and weight.dtype == torch.bfloat16 and ids.dtype == torch.int64
+            and mg.dtype == torch.float32 and mg.is_contiguous() and mg.shape == weight.shape and mg.data_ptr() % 16 == 0
+            and weight.shape[1] % 8 == 0):
+        return _EmbeddingFn.apply(ids, weight, mg)
+    return torch.nn.functional.embedding(ids, weight)
+
+
 # ------------------------------------------------------------------------------------------------ RoPE
 def mrope_tables(pos3: torch.Tensor, theta: float, rot: int, sections, interleaved_sections: bool = True):
     """Multi-axis rotary tables.  ``pos3`` [T, 3] = (temporal, height, width) index of every token; frequency ``i``

@@ -9,6 +9,8 @@ from __future__ import annotations
 import torch
 import torch.distributed as dist
 
+from ..ops import fused
+
 
 def _ws(group):
     return dist.get_world_size(group) if (group is not None and dist.is_initialized()) else 1
@@ -246,5 +248,5 @@ def vocab_parallel_embedding(ids, weight, vocab_start, group):
     """Embedding lookup with the table sharded over the vocabulary; out-of-shard ids contribute zero and the
     partial rows are summed over the TP group."""
     if _ws(group) == 1:
-        return torch.nn.functional.embedding(ids, weight)
+        return fused.embedding(ids, weight)
     return _VocabParallelEmbedding.apply(ids, weight, vocab_start, group)
