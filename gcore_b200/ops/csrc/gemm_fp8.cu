@@ -3,25 +3,32 @@
 // (the DeepSeek-V3 recipe; the reference's TileLang version is gfused/mygemm_fp8.py:45-97).
 //
 // Two-level accumulation: every 128-deep K block is multiplied on the tensor core into a fresh TMEM accumulator
-// (four buffers in rotation); eight promotion warps (two per TMEM lane quarter, 64 columns each) pull that partial
+// (in rotation); eight promotion warps (two per TMEM lane quarter, half of the columns each) pull that partial
 // product out of TMEM, apply sA * sB and add it into fp32 register accumulators while the tensor core already works
-// on the next block.  The promotion has to keep up with ~270 tensor-core cycles per block, hence the eight warps,
-// both TMEM loads of a thread in flight at once and the scales fetched one block ahead.  bf16 or fp32 output.
+// on the next block, with the scales fetched one block ahead.  bf16 or fp32 output.
+//
+// What bounds it is the operands' way from L2: 128 x 128 tiles need a byte per 128 operations, 10 TB/s at 1.28 PFLOP/s,
+// which is where they stop.  128 x 256 tiles need a quarter less; their register accumulators (128 per promotion thread) are
+// the most the register file holds.  us, narrow -> wide: 3400 x 36864 x 7168 1362 -> 1055 (1.70 PFLOP/s), 3400 x 7168 x 16384
+// 643 -> 531, 3400 x 24576 x 1536 252 -> 222, 8192^3 840 -> 678 (1.62).
 #include "ptx.cuh"
 #include "host_utils.h"
 
 namespace gk8 {
 using namespace gk;
 
-constexpr int BM = 128, BN = 128, BK = 128;  // BK bytes = 128 = one swizzle row of e4m3
+constexpr int BM = 128, BK = 128;  // BK bytes = 128 = one swizzle row of e4m3
 constexpr int UMMA_K = 32;
-constexpr int STAGES = 5;
 constexpr int THREADS = 320;          // TMA warp, MMA warp, 8 promotion warps
 constexpr int PROMO_THREADS = 256;
-constexpr int HALF = BN / 2;           // columns per promotion warp
-constexpr int NBUF = 4;                // TMEM accumulators in flight (4 x 128 columns = all of TMEM)
-constexpr int STAGE_BYTES = (BM + BN) * BK;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+template <int BN>
+struct Cfg8 {
+  static constexpr int HALF = BN / 2;     // columns per promotion warp
+  static constexpr int NBUF = 512 / BN;   // TMEM accumulators in flight (all of TMEM)
+  static constexpr int STAGES = BN == 128 ? 5 : 4;
+  static constexpr int STAGE_BYTES = (BM + BN) * BK;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+};
 
 struct P8 {
   int M, N, K;
@@ -49,8 +56,10 @@ __device__ __forceinline__ int group_of(const P8& p, int m0) {
   return lo;
 }
 
+template <int BN>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, P8 p) {
+  constexpr int HALF = Cfg8<BN>::HALF, NBUF = Cfg8<BN>::NBUF, STAGES = Cfg8<BN>::STAGES, STAGE_BYTES = Cfg8<BN>::STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
@@ -138,11 +147,13 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
     const int m0 = (tile % mt) * BM, n0 = (tile / mt) * BN;
     const int row = m0 + quad * 32 + lane;
-    int nb = n0 / 128;
+    const int nbs = (p.N + 127) / 128;
+    int nb = (n0 + half * HALF) / 128;       // a warp's columns share one block of weight scales
+    if (nb >= nbs) nb = nbs - 1;             // columns behind the last one are not stored
     if (p.group_offsets) {
       const int g = group_of(p, m0);
       if (g < 0) continue;
-      nb += g * ((p.N + 127) / 128);
+      nb += g * nbs;
     }
     float acc[HALF];
 #pragma unroll
@@ -158,16 +169,31 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       if (!ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + a * BN + half * HALF;
-      uint32_t r0[32], r1[32];
-      tmem_ld32(taddr, r0);
-      tmem_ld32(taddr + 32, r1);
-      tmem_ld_wait();
-      tc_fence_before();
-      mbar_arrive(&tempty[a]);                 // the values are in registers: the buffer can take the next block
+      if constexpr (HALF == 64) {
+        uint32_t r0[32], r1[32];
+        tmem_ld32(taddr, r0);
+        tmem_ld32(taddr + 32, r1);
+        tmem_ld_wait();
+        tc_fence_before();
+        mbar_arrive(&tempty[a]);                 // the values are in registers: the buffer can take the next block
 #pragma unroll
-      for (int j = 0; j < 32; ++j) acc[j] = fmaf(sc, __uint_as_float(r0[j]), acc[j]);
+        for (int j = 0; j < 32; ++j) acc[j] = fmaf(sc, __uint_as_float(r0[j]), acc[j]);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) acc[32 + j] = fmaf(sc, __uint_as_float(r1[j]), acc[32 + j]);
+        for (int j = 0; j < 32; ++j) acc[32 + j] = fmaf(sc, __uint_as_float(r1[j]), acc[32 + j]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < HALF / 32; ++c) {
+          uint32_t r0[32];
+          tmem_ld32(taddr + c * 32, r0);
+          tmem_ld_wait();
+          if (c == HALF / 32 - 1) {
+            tc_fence_before();
+            mbar_arrive(&tempty[a]);
+          }
+#pragma unroll
+          for (int j = 0; j < 32; ++j) acc[c * 32 + j] = fmaf(sc, __uint_as_float(r0[j]), acc[c * 32 + j]);
+        }
+      }
     }
     if (ok && row < p.M) {
 #pragma unroll
@@ -207,34 +233,45 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
 using namespace gk8;
 
+template <int BN>
+static int launch_fp8(const void* A, long long lda, long long a_rows, const void* B, long long ldb, long long b_rows, const P8& p,
+                      cudaStream_t st) {
+  CUtensorMap tmA, tmB;
+  if (gk::make_tmap_2d(&tmA, A, 1, a_rows, p.K, lda, BM, BK, true)) return -2;
+  if (gk::make_tmap_2d(&tmB, B, 1, b_rows, p.K, ldb, BN, BK, true)) return -3;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(gemm_fp8_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg8<BN>::SMEM_BYTES) !=
+        cudaSuccess)
+      return -4;
+    configured = true;
+  }
+  const long long tiles = static_cast<long long>((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+  const int sms = gk::sm_count();
+  gemm_fp8_kernel<BN><<<static_cast<unsigned>(tiles < sms ? tiles : sms), THREADS, Cfg8<BN>::SMEM_BYTES, st>>>(tmA, tmB, p);
+  return gk::launch_status();
+}
+
+// A wide tile is twice the work at four thirds of the rate: 1.5 narrow ones.  With few K blocks per tile the store counts, which
+// two warps per lane quarter do for twice the columns (3400 x 32768 x 512: 158 us against 147).
+static bool wide_tiles_pay(int M, int N, int K) {
+  if (K < 1024) return false;
+  const long long mt = (M + BM - 1) / BM, sms = gk::sm_count();
+  const long long narrow = (mt * ((N + 127) / 128) + sms - 1) / sms, wide = (mt * ((N + 255) / 256) + sms - 1) / sms;
+  return 3 * wide <= 2 * narrow;
+}
+
 // A [M,K] and B [N,K] are e4m3 bytes (row-major, K contiguous, K % 16 == 0); sA fp32 [M, ceil(K/128)],
 // sB fp32 [ceil(N/128), ceil(K/128)].
 GK_EXPORT int gk_gemm_fp8_blockscaled(const void* A, long long lda, const void* B, long long ldb, const float* sA,
                                       const float* sB, void* C, long long ldc, int out_fp32, int M, int N, int K,
                                       int* err, void* stream) {
   if ((lda & 15) || (ldb & 15) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -1;
-  CUtensorMap tmA, tmB;
-  if (gk::make_tmap_2d(&tmA, A, 1, M, K, lda, BM, BK, true)) return -2;
-  if (gk::make_tmap_2d(&tmB, B, 1, N, K, ldb, BN, BK, true)) return -3;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
-      return -4;
-    configured = true;
-  }
   P8 p;
   p.M = M; p.N = N; p.K = K; p.sA = sA; p.sB = sB; p.C = C; p.ldc = ldc; p.out_fp32 = out_fp32; p.err = err;
   p.group_offsets = nullptr; p.num_groups = 0;
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
-  }
-  gemm_fp8_kernel<<<tiles < sms ? tiles : sms, THREADS, SMEM_BYTES, reinterpret_cast<cudaStream_t>(stream)>>>(tmA, tmB, p);
-  return gk::launch_status();
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  return wide_tiles_pay(M, N, K) ? launch_fp8<256>(A, lda, M, B, ldb, N, p, st) : launch_fp8<128>(A, lda, M, B, ldb, N, p, st);
 }
 
 // Ragged-M grouped form (experts): A [M_cap, K] e4m3 with expert-sorted rows, group g = rows [offsets[g],
@@ -245,20 +282,11 @@ GK_EXPORT int gk_gemm_fp8_grouped(const void* A, long long lda, const void* B, l
                                   const int* offsets, int num_groups, int* err, void* stream) {
   if ((lda & 15) || (ldb & 15) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -1;
   if (num_groups < 1 || !offsets || M_cap % BM) return -5;
-  CUtensorMap tmA, tmB;
-  if (gk::make_tmap_2d(&tmA, A, 1, M_cap, K, lda, BM, BK, true)) return -2;
-  if (gk::make_tmap_2d(&tmB, B, 1, static_cast<uint64_t>(num_groups) * N, K, ldb, BN, BK, true)) return -3;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
-      return -4;
-    configured = true;
-  }
   P8 p;
   p.M = M_cap; p.N = N; p.K = K; p.sA = sA; p.sB = sB; p.C = C; p.ldc = ldc; p.out_fp32 = out_fp32; p.err = err;
   p.group_offsets = offsets; p.num_groups = num_groups;
-  const int tiles = (M_cap / BM) * ((N + BN - 1) / BN);
-  const int sms = gk::sm_count();
-  gemm_fp8_kernel<<<tiles < sms ? tiles : sms, THREADS, SMEM_BYTES, reinterpret_cast<cudaStream_t>(stream)>>>(tmA, tmB, p);
-  return gk::launch_status();
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const long long b_rows = static_cast<long long>(num_groups) * N;
+  return wide_tiles_pay(M_cap, N, K) ? launch_fp8<256>(A, lda, M_cap, B, ldb, b_rows, p, st)
+                                  : launch_fp8<128>(A, lda, M_cap, B, ldb, b_rows, p, st);
 }
