@@ -309,6 +309,7 @@ def linear_forward(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None =
     from HBM exactly once with every SM busy."""
     T, K = x.shape
     N = w.shape[0]
+    assert w.shape[1] == K, f"contraction mismatch {K} vs {w.shape[1]}"   # the decode kernels take K from x alone
     if x.is_cuda and x.dtype == torch.float32:
         return _linear_f32(x, w, bias, out)
     if _lib.use_native(x) and T <= 128 and N >= 256:

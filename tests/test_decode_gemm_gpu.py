@@ -71,3 +71,12 @@ def test_streams_and_captured_branches_keep_their_counters_apart():
         torch.cuda.synchronize()
         assert torch.equal(a, ref[0]) and torch.equal(b, ref[1])
     _lib.check_device_errors()
+
+
+@pytest.mark.parametrize("N,K", [(3584, 4096), (1024, 512)])
+def test_refuses_a_weight_of_another_width(N, K):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    w = torch.zeros(N, K, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(AssertionError, match="contraction mismatch"):
+        G.linear_forward(w[:4, :K - 64].contiguous(), w)
