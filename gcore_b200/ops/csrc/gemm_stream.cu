@@ -19,9 +19,6 @@
 // columns each).  Two accumulators: a piece is drained while the next one is contracted.
 #include "ptx.cuh"
 #include "host_utils.h"
-#include <map>
-#include <mutex>
-#include <utility>
 
 namespace gkst {
 using namespace gk;
@@ -317,60 +314,26 @@ static int padded_tokens(int T) { return (T + 15) / 16 * 16; }
 
 using namespace gkst;
 
-// Counters of the divided tiles.  A launch leaves them at zero; launches that may run at the same time must not share them:
-// every stream has a slot of its own, and so has every stream of a capture (a graph may be replayed anywhere).  Captures
-// take the upper half of the slots in turn, streams the lower half.  The buffer is the caller's (one per device, zeroed).
-namespace {
-struct CounterPool {
-  int* base = nullptr;
-  int slots = 0, ints = 0, next[2] = {0, 0};
-  std::map<std::pair<unsigned long long, cudaStream_t>, int> taken;   // (capture, 0 outside of one; stream) -> slot
-};
-std::mutex pools_mutex;
-std::map<int, CounterPool> pools;   // by device
-
-int* counters_of(cudaStream_t st, int need) {
-  int dev = 0;
+// Id of the capture that a stream takes part in, 0 outside of one (or where it cannot be told).
+GK_EXPORT unsigned long long gk_capture_id(void* stream) {
   cudaStreamCaptureStatus status;
   unsigned long long id = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) {
+  if (cudaStreamGetCaptureInfo(reinterpret_cast<cudaStream_t>(stream), &status, &id) != cudaSuccess) {
     cudaGetLastError();
-    return nullptr;
+    return 0;
   }
-  const int half = status == cudaStreamCaptureStatusActive ? 1 : 0;
-  std::lock_guard<std::mutex> lock(pools_mutex);
-  CounterPool& pool = pools[dev];
-  if (!pool.base || pool.ints < need) return nullptr;
-  if (pool.taken.size() >= 4u * pool.slots) pool.taken.clear();
-  auto [it, fresh] = pool.taken.try_emplace({half ? id : 0ull, st}, 0);
-  if (fresh) {
-    it->second = pool.next[half] + half * (pool.slots / 2);
-    pool.next[half] = (pool.next[half] + 1) % (pool.slots / 2);
-  }
-  return pool.base + static_cast<long long>(it->second) * pool.ints;
-}
-}  // namespace
-
-// The current device's counters: `slots` (even) times `ints` (even) zeroed ints, 8-byte aligned.
-GK_EXPORT int gk_gemm_stream_pool(int* base, int slots, int ints) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || slots < 2 || slots % 2 || ints % 2 || (reinterpret_cast<uintptr_t>(base) & 7)) return -1;
-  std::lock_guard<std::mutex> lock(pools_mutex);
-  CounterPool& pool = pools[dev];
-  pool.base = base; pool.slots = slots; pool.ints = ints;
-  pool.next[0] = pool.next[1] = 0;
-  pool.taken.clear();
-  return 0;
+  return status == cudaStreamCaptureStatusActive ? id : 0;
 }
 
 // Floats of scratch for the pieces of divided tiles.
 GK_EXPORT long long gk_gemm_stream_scratch(int T) { return 2ll * sm_count() * padded_tokens(T) * BM; }
 
-// W [N, K] and X [T, K] bf16 row-major (K contiguous, leading dimensions multiples of 8, 16-byte aligned), 1 <= T <= 128;
-// the device's pool of counters has to hold two per 128 features in a slot (-9 without).
+// W [N, K] and X [T, K] bf16 row-major (K contiguous, leading dimensions multiples of 8, 16-byte aligned), 1 <= T <= 128.
+// counters: two zero ints per 128 features, 8-byte aligned; a launch leaves them at zero, and launches that may run at the
+// same time must not share them.
 GK_EXPORT int gk_gemm_stream(const void* W, long long ldw, const void* X, long long ldx, void* Y, long long ldy,
                              int out_fp32, const void* bias, int bias_fp32, int T, int N, int K, float* ws,
-                             long long ws_floats, int* err, void* stream) {
+                             long long ws_floats, int* counters, long long counter_ints, int* err, void* stream) {
   if (T < 1 || T > 128 || N < 1 || K < 1) return -1;
   if ((ldw & 7) || (ldx & 7) || (reinterpret_cast<uintptr_t>(W) & 15) || (reinterpret_cast<uintptr_t>(X) & 15)) return -3;
   StParams p;
@@ -380,8 +343,7 @@ GK_EXPORT int gk_gemm_stream(const void* W, long long ldw, const void* X, long l
   if (static_cast<long long>(tiles) * p.kbs > 0x3fffffff) return -2;
   p.units = tiles * p.kbs;
   if (ws_floats < gk_gemm_stream_scratch(T)) return -8;
-  int* counters = counters_of(reinterpret_cast<cudaStream_t>(stream), 2 * tiles);
-  if (!counters) return -9;
+  if (!counters || counter_ints < 2ll * tiles || (reinterpret_cast<uintptr_t>(counters) & 7)) return -9;
   CUtensorMap tmW, tmX;
   if (make_tmap_2d(&tmW, W, 2, N, K, ldw, BM, BK, true)) return -4;
   if (make_tmap_2d(&tmX, X, 2, T, K, ldx, p.Tp, BK, true)) return -5;

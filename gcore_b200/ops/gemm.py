@@ -273,23 +273,30 @@ def _skinny_plan(T: int, tiles: int, kb: int, K: int):
 
 
 STREAM = {"enabled": os.environ.get("GCORE_STREAM_GEMM", "1") != "0"}
-COUNTER_SLOTS, SLOT_INTS = 256, 8192
-_COUNTERS: dict = {}        # device index -> zeroed counters of all slots
 _STREAM_SCRATCH: dict = {}  # tokens -> floats of scratch
+COUNTER_INTS, COUNTER_OWNERS = 8192, 64
+_COUNTERS: dict = {}   # (device, stream) -> counters of divided tiles, zero between launches
+_CAPTURED: dict = {}   # (device, stream, capture) -> the same in a capture under way
 
 
-def _stream_ready(device, N: int) -> bool:
-    """Gives the library its zeroed counters on a device's first use.  False inside a capture (they cannot be made there)
-    and for more tiles than a slot counts."""
-    if device.index not in _COUNTERS:
-        if torch.cuda.is_current_stream_capturing():
-            return False
-        counters = torch.zeros(COUNTER_SLOTS, SLOT_INTS, dtype=torch.int32, device=device)
-        torch.cuda.current_stream(device).synchronize()   # once: other streams use it without waiting for this one
-        with torch.cuda.device(device):
-            _lib.check(_lib.kernels().gk_gemm_stream_pool(_lib.ptr(counters), COUNTER_SLOTS, SLOT_INTS), "gemm_stream_pool")
-        _COUNTERS[device.index] = counters
-    return (N + 127) // 128 * 2 <= SLOT_INTS
+def _counters(lib, device, stream, N: int) -> torch.Tensor:
+    """Zeroed counters for a launch on the current stream ``stream`` of ``device``.  Launches that may overlap do not share
+    them: every stream has its own, and so has every stream of a capture (a graph may be replayed anywhere, so it clears
+    its own each time).  They are allocated on their stream, so that one which is dropped here is only written again behind
+    the launches that hold it."""
+    ints = (N + 127) // 128 * 2
+    if torch.cuda.is_current_stream_capturing():
+        owners, key = _CAPTURED, (device.index, stream.value, lib.gk_capture_id(stream))
+    else:
+        if _CAPTURED:
+            _CAPTURED.clear()   # what a finished capture leaves here would keep its pool's memory
+        owners, key = _COUNTERS, (device.index, stream.value)
+    counters = owners.get(key)
+    if counters is None or counters.numel() < ints:
+        if len(owners) >= COUNTER_OWNERS:
+            owners.clear()
+        counters = owners[key] = torch.zeros(max(ints, COUNTER_INTS), dtype=torch.int32, device=device)
+    return counters
 
 
 def _linear_f32(x, w, bias, out):
@@ -320,20 +327,19 @@ def linear_forward(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None =
                 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
                 and (out is None or (out.dtype in (torch.bfloat16, torch.float32) and out.stride(1) == 1))
                 and (out is not None or (out_dtype or x.dtype) in (torch.bfloat16, torch.float32))):
-            if _stream_ready(x.device, N):
-                lib = _lib.kernels()
-                y = out if out is not None else torch.empty((T, N), dtype=out_dtype or x.dtype, device=x.device)
-                floats = _STREAM_SCRATCH.get(T)
-                if floats is None:
-                    floats = _STREAM_SCRATCH[T] = lib.gk_gemm_stream_scratch(T)
-                ws = torch.empty(floats, dtype=torch.float32, device=x.device)
-                LAUNCHES["gemm"] += 1
-                rc = lib.gk_gemm_stream(
-                    w.data_ptr(), w.stride(0), x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0),
-                    y.dtype == torch.float32, _lib.ptr(bias), bias is not None and bias.dtype == torch.float32, T, N, K,
-                    ws.data_ptr(), floats, _lib.err_flag(x.device).data_ptr(), _lib.stream_ptr())
-                _lib.check(rc, "gk_gemm_stream")
-                return y
+            lib, stream = _lib.kernels(), _lib.stream_ptr()
+            y = out if out is not None else torch.empty((T, N), dtype=out_dtype or x.dtype, device=x.device)
+            floats = _STREAM_SCRATCH.get(T)
+            if floats is None:
+                floats = _STREAM_SCRATCH[T] = lib.gk_gemm_stream_scratch(T)
+            ws, counters = torch.empty(floats, dtype=torch.float32, device=x.device), _counters(lib, x.device, stream, N)
+            LAUNCHES["gemm"] += 1
+            rc = lib.gk_gemm_stream(
+                w.data_ptr(), w.stride(0), x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0),
+                y.dtype == torch.float32, _lib.ptr(bias), bias is not None and bias.dtype == torch.float32, T, N, K,
+                ws.data_ptr(), floats, counters.data_ptr(), counters.numel(), _lib.err_flag(x.device).data_ptr(), stream)
+            _lib.check(rc, "gk_gemm_stream")
+            return y
         bn = 32 if T <= 32 else (64 if T <= 64 else 128)
         tiles = (N + 127) // 128
         kb = (K + 63) // 64

@@ -80,3 +80,68 @@ def test_refuses_a_weight_of_another_width(N, K):
     w = torch.zeros(N, K, device="cuda", dtype=torch.bfloat16)
     with pytest.raises(AssertionError, match="contraction mismatch"):
         G.linear_forward(w[:4, :K - 64].contiguous(), w)
+
+
+def _problem(seed, n=2):
+    T, N, K = 8, 3584, 4096
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    xs = [torch.randn(T, K, generator=g, device="cuda").bfloat16() for _ in range(n)]
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    return xs, w, [G.linear_forward(x, w, out_dtype=torch.float32) for x in xs]
+
+
+def test_no_two_live_graphs_share_counters(monkeypatch):
+    """More captures than a fixed table would hold; the first and the last graph at once on two streams."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    xs, w, ref = _problem(5)
+    own, seen = G._counters, []
+    monkeypatch.setattr(G, "_counters", lambda *a: (lambda c: (seen.append(c.data_ptr()), c)[1])(own(*a)))
+    graphs, outs = [], []
+    for i in range(132):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs.append([G.linear_forward(xs[i % 2], w, out_dtype=torch.float32) for _ in range(2)])
+        graphs.append(graph)
+    assert len(seen) == 264 and len(set(seen)) == 132       # one for both products of a capture
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for _ in range(50):
+        for s, graph in zip(streams, (graphs[0], graphs[-1])):
+            with torch.cuda.stream(s):
+                graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, ref[0]) for y in outs[0]) and all(torch.equal(y, ref[1]) for y in outs[-1])
+    G.linear_forward(xs[0], w)
+    assert not G._CAPTURED                                   # nothing keeps a finished capture's memory
+    _lib.check_device_errors()
+
+
+def test_first_use_in_a_capture_and_in_two_threads(monkeypatch):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    import threading
+    xs, w, ref = _problem(6)
+    G._COUNTERS.clear()
+    graph = torch.cuda.CUDAGraph()
+    before = G.LAUNCHES["gemm"]
+    with torch.cuda.graph(graph):
+        y = G.linear_forward(xs[0], w, out_dtype=torch.float32)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, ref[0]) and G.LAUNCHES["gemm"] == before + 1   # the same kernel as outside
+    monkeypatch.setattr(G, "COUNTER_OWNERS", 1)              # owners push one another out all the time
+    outs, go = [[], []], threading.Barrier(2)
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            go.wait()
+            for _ in range(100):
+                outs[i].append(G.linear_forward(xs[i], w, out_dtype=torch.float32))
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert all(len(o) == 100 and all(torch.equal(y, r) for y in o) for o, r in zip(outs, ref))
+    _lib.check_device_errors()
