@@ -125,6 +125,9 @@ def err_flag(device) -> torch.Tensor:
     return _ERR_FLAGS[idx]
 
 
+ON_DEVICE_ERROR: list = []   # called before a reported error is raised: state that a kernel which gave up left behind
+
+
 def check_device_errors(device=None):
     """Synchronising check of the kernel error word; raises if any kernel gave up on a wait."""
     if not torch.cuda.is_available():
@@ -135,6 +138,8 @@ def check_device_errors(device=None):
         code = int(_ERR_FLAGS[idx].item())
         if code != 0:
             _ERR_FLAGS[idx].zero_()
+            for reset in ON_DEVICE_ERROR:
+                reset()
             raise RuntimeError(f"gcore_b200 kernel reported a timed-out wait (code {code})")
 
 

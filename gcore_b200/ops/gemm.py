@@ -299,6 +299,10 @@ def _counters(lib, device, stream, N: int) -> torch.Tensor:
     return counters
 
 
+# a launch that gave up on a wait leaves its counters at what they were; graphs clear theirs at every replay
+_lib.ON_DEVICE_ERROR.append(_COUNTERS.clear)
+
+
 def _linear_f32(x, w, bias, out):
     """32-bit models: the library's true fp32 product (never TF32)."""
     tf32 = torch.backends.cuda.matmul.allow_tf32

@@ -145,3 +145,24 @@ def test_first_use_in_a_capture_and_in_two_threads(monkeypatch):
     [t.join() for t in threads]
     assert all(len(o) == 100 and all(torch.equal(y, r) for y in o) for o, r in zip(outs, ref))
     _lib.check_device_errors()
+
+
+def test_counters_start_over_after_a_reported_error():
+    """What a launch that gave up leaves behind: counters that are not zero, on every stream and inside a graph."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    xs, w, ref = _problem(7)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = G.linear_forward(xs[1], w, out_dtype=torch.float32)
+        captured = list(G._CAPTURED.values())
+    for c in list(G._COUNTERS.values()) + captured:
+        c.fill_(3)
+    torch.cuda.synchronize()
+    _lib.err_flag(w.device).fill_(1)
+    with pytest.raises(RuntimeError, match="timed-out wait"):
+        _lib.check_device_errors()
+    for _ in range(3):
+        graph.replay()
+        assert torch.equal(y, ref[1]) and torch.equal(G.linear_forward(xs[0], w, out_dtype=torch.float32), ref[0])
+    _lib.check_device_errors()
