@@ -65,6 +65,9 @@ class Router(nn.Module):
         if self.lora is not None:
             logits = logits + self.lora(x.float())
         replay = RouterReplay.get(self.layer_idx) if RouterReplay.mode == "replay" else None
+        if replay is not None:
+            # forced ids become row numbers of the token-movement kernels, which do not look at their range again
+            torch._assert_async(((replay >= 0) & (replay < E)).all(), "replayed expert id out of range")
         from ..ops.router import route
         sigmoid = cfg.moe_router_type != "softmax"
         idx, w = route(logits, self.expert_bias if sigmoid else None, replay, K, cfg.moe_n_group if sigmoid else 1,

@@ -873,3 +873,23 @@ def test_fp8_data_and_weight_gradients_follow_the_bf16_ones(monkeypatch):
             torch.randn(384, 128, generator=torch.Generator().manual_seed(7)))
         outs.append(x.grad)
     assert not torch.equal(outs[0], outs[1]) and (outs[0] - outs[1]).abs().max() / outs[0].abs().max() < 0.08
+
+
+@pytest.mark.parametrize("bad", [-1, 8])
+def test_replayed_expert_ids_are_checked_before_they_become_row_numbers(bad, monkeypatch):
+    """The native routing kernel passes forced ids on as they are (stood in for here); what follows indexes with them."""
+    from gcore_b200.models.config import ModelConfig
+    from gcore_b200.models.moe import Router, RouterReplay
+    monkeypatch.setattr("gcore_b200.ops.router.route", lambda logits, bias, replay, *a: (replay, torch.zeros(replay.shape)))
+    router = Router(ModelConfig(arch="qwen3_moe", num_layers=1, hidden_size=16, num_attention_heads=2, num_kv_heads=2,
+                                ffn_hidden_size=16, vocab_size=32, num_experts=8, moe_top_k=2, moe_ffn_hidden_size=16), 0)
+    torch.nn.init.zeros_(router.weight)
+    ids = torch.tensor([[0, 7], [3, 4], [6, 1]])
+    try:
+        RouterReplay.set("replay", {0: ids})
+        assert torch.equal(router(torch.zeros(3, 16))[0], ids)
+        ids[1, 1] = bad
+        with pytest.raises(RuntimeError, match="out of range"):
+            router(torch.zeros(3, 16))
+    finally:
+        RouterReplay.set("off")
