@@ -123,6 +123,22 @@ __device__ __forceinline__ void sum_pieces(const StParams& p, int tile, int lo, 
   }
 }
 
+// The epilogue warps meet at barriers behind a divided tile: where one of them has given up on a wait, all leave together.
+__device__ __forceinline__ bool all_epilogue_warps(bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 p, %1, 0;\n"
+      "barrier.red.and.pred q, 1, %2, p;\n"
+      "selp.u32 %0, 1, 0, q;\n"
+      "}\n"
+      : "=r"(all)
+      : "r"(static_cast<uint32_t>(ok)), "n"(EPI_THREADS)
+      : "memory");
+  return all != 0;
+}
+
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
 
 // What follows when this CTA's piece of a divided tile lies in the scratch.
@@ -213,12 +229,10 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (warp == 0) {
     const int pre = u1 - u0 < p.stages ? u1 - u0 : p.stages;
     int tile = u0 / p.kbs, kb = u0 - tile * p.kbs;
-    int s = 0;
+    int s = 0, i = 0;
     uint32_t ph = 0;
-    bool ok = true;
-    for (int i = 0; i < u1 - u0 && ok; ++i) {
-      if (i >= pre) ok = mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY);
-      if (!ok) break;
+    for (; i < u1 - u0; ++i) {
+      if (i >= pre && !mbar_wait_warp(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY)) break;
       if (lane == 0) {
         uint8_t* sa = smem + s * stage_bytes;
         if (i >= pre) {
@@ -231,16 +245,16 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       if (++kb == p.kbs) { kb = 0; ++tile; }
       if (++s == p.stages) { s = 0; ph ^= 1; }
     }
+    for (int j = i > p.stages ? i - p.stages : 0; j < i; ++j) mbar_land(&full[j % p.stages], (j / p.stages) & 1);
   } else if (warp == 1) {
     const uint32_t idesc = make_idesc(BM, p.Tp, 1, 1, 0, 0);
-    int s = 0, piece = 0, kb = u0 % p.kbs;
+    int s = 0, piece = 0, kb = u0 % p.kbs, u = u0;
     uint32_t ph = 0;
-    bool ok = true, fresh = true;
-    for (int u = u0; u < u1 && ok; ++u) {
+    bool fresh = true;
+    for (; u < u1; ++u) {
       const int acc = piece & 1;
-      if (fresh) ok = mbar_wait(&tempty[acc], ((piece >> 1) & 1) ^ 1, p.err, ERR_WAIT_TMEM_EMPTY);
-      if (ok) ok = mbar_wait(&full[s], ph, p.err, ERR_WAIT_FULL);
-      if (!ok) break;
+      if (fresh && !mbar_wait_warp(&tempty[acc], ((piece >> 1) & 1) ^ 1, p.err, ERR_WAIT_TMEM_EMPTY)) break;
+      if (!mbar_wait_warp(&full[s], ph, p.err, ERR_WAIT_FULL)) break;
       tc_fence_after();
       const bool ends = kb == p.kbs - 1 || u == u1 - 1;
       if (lane == 0) {
@@ -259,20 +273,20 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       if (++kb == p.kbs) kb = 0;
       if (++s == p.stages) { s = 0; ph ^= 1; }
     }
+    const int last = u - u0 - 1;   // the products of the last k-block, and with them all before
+    if (last >= 0) mbar_land(&empty[last % p.stages], (last / p.stages) & 1);
   } else {
     const int quad = warp & 3;
     const int row = quad * 32 + lane;                // output feature inside the tile = TMEM lane
     const int half = (warp - 2) >> 2;                // which token columns
     const int c0 = half * (p.Tp / 2), c1 = c0 + p.Tp / 2;
-    bool ok = true;
     int piece = 0;
-    for (int u = u0; u < u1 && ok; ++piece) {
+    for (int u = u0; u < u1; ++piece) {
       const int tile = u / p.kbs, kb0 = u - tile * p.kbs;
       const int next = (tile + 1) * p.kbs < u1 ? (tile + 1) * p.kbs : u1;
       const bool whole = kb0 == 0 && next - u == p.kbs;
       const int acc = piece & 1, feat = tile * BM + row;
-      ok = mbar_wait(&tfull[acc], (piece >> 1) & 1, p.err, ERR_WAIT_TMEM_FULL);
-      if (!ok) break;
+      if (!all_epilogue_warps(mbar_wait(&tfull[acc], (piece >> 1) & 1, p.err, ERR_WAIT_TMEM_FULL))) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * p.Tp + (static_cast<uint32_t>(quad * 32) << 16);
       float bias = 0.f;

@@ -103,14 +103,14 @@ moe_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   const int ftiles = (p.F + FT - 1) / FT, ntiles = s_off[p.E] / SEG * ftiles, kbs = (p.K + BK - 1) / BK;
 
   if (warp == 0) {
-    int s = 0;
+    int s = 0, fills = 0;
     uint32_t ph = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
       const Tile t = tile_at(s_off, p, tile, ftiles);
       const int w0 = t.expert * p.N + t.f * FT, w1 = ACT ? w0 + p.F : w0 + 64;
       for (int kb = 0; kb < kbs; ++kb) {
-        ok = mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY);
+        ok = mbar_wait_warp(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY);
         if (!ok) break;
         if (lane == 0) {
           uint8_t* sa = smem + s * STAGE_BYTES;
@@ -120,21 +120,23 @@ moe_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           tma_load_2d(sa + A_BYTES, &tmX, &full[s], kb * BK, t.row0);
         }
         __syncwarp();
+        ++fills;
         if (++s == STAGES) { s = 0; ph ^= 1; }
       }
     }
+    for (int j = fills > STAGES ? fills - STAGES : 0; j < fills; ++j) mbar_land(&full[j % STAGES], (j / STAGES) & 1);
   } else if (warp == 1) {
     constexpr uint32_t idesc = make_idesc(BM, SEG, 1, 1, 0, 0);
-    int s = 0, n = 0;
+    int s = 0, n = 0, used = 0;
     uint32_t ph = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++n) {
       const int acc = n & 1;
-      ok = mbar_wait(&tempty[acc], ((n >> 1) & 1) ^ 1, p.err, ERR_WAIT_TMEM_EMPTY);
+      ok = mbar_wait_warp(&tempty[acc], ((n >> 1) & 1) ^ 1, p.err, ERR_WAIT_TMEM_EMPTY);
       if (!ok) break;
       tc_fence_after();
       for (int kb = 0; kb < kbs; ++kb) {
-        ok = mbar_wait(&full[s], ph, p.err, ERR_WAIT_FULL);
+        ok = mbar_wait_warp(&full[s], ph, p.err, ERR_WAIT_FULL);
         if (!ok) break;
         tc_fence_after();
         if (lane == 0) {
@@ -147,9 +149,11 @@ moe_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           if (kb == kbs - 1) umma_commit(&tfull[acc]);
         }
         __syncwarp();
+        ++used;
         if (++s == STAGES) { s = 0; ph ^= 1; }
       }
     }
+    if (used) mbar_land(&empty[(used - 1) % STAGES], ((used - 1) / STAGES) & 1);   // the last products, and all before
   } else {
     const int quad = warp & 3, row = quad * 32 + lane;    // weight row inside the tile = TMEM lane
     int n = 0;
@@ -157,7 +161,7 @@ moe_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++n) {
       const Tile t = tile_at(s_off, p, tile, ftiles);
       const int acc = n & 1;
-      ok = mbar_wait(&tfull[acc], (n >> 1) & 1, p.err, ERR_WAIT_TMEM_FULL);
+      ok = mbar_wait_warp(&tfull[acc], (n >> 1) & 1, p.err, ERR_WAIT_TMEM_FULL);
       if (ACT) ok = all_epilogue_warps(ok);   // the four warps meet at barriers: they leave the loop together
       if (!ok) break;
       tc_fence_after();

@@ -88,6 +88,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   return true;
 }
 
+// The same answer for every lane of the calling warp, so that its lanes leave a loop together.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* err, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, code)) != 0;
+}
+// Waits for copies or products under way, whether or not a role has failed: a CTA that gives up must not hand back shared or
+// tensor memory that they still use.  Bounded too (about 10 ms).
+constexpr long long LAND_BUDGET_CYCLES = 20000000LL;
+__device__ __forceinline__ void mbar_land(uint64_t* bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity))
+    if (clock64() - t0 > LAND_BUDGET_CYCLES) return;
+}
+
 // ---------------------------------------------------------------- TMA (never multicast)
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

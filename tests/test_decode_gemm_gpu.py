@@ -166,3 +166,21 @@ def test_counters_start_over_after_a_reported_error():
         graph.replay()
         assert torch.equal(y, ref[1]) and torch.equal(G.linear_forward(xs[0], w, out_dtype=torch.float32), ref[0])
     _lib.check_device_errors()
+
+
+@pytest.mark.parametrize("N,K", [(3584, 3584), (24576, 512), (32768, 520)])
+def test_ends_while_an_earlier_error_stands(N, K):
+    """Another kernel's error makes waits give up early: the launch ends, and the one after the report is right."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(8, K, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    ref = G.linear_forward(x, w, out_dtype=torch.float32)
+    for _ in range(5):
+        _lib.err_flag(w.device).fill_(1)
+        G.linear_forward(x, w)
+        with pytest.raises(RuntimeError, match="timed-out wait"):
+            _lib.check_device_errors()
+        assert torch.equal(G.linear_forward(x, w, out_dtype=torch.float32), ref)
+    _lib.check_device_errors()
