@@ -492,7 +492,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       const int row = t.m0 + row_in_tile;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
-      if (MINB == 1 && p.staged) {
+      // a ragged-M segment that ends inside these 32 rows: the threads store its rows, the next segment's are not touched
+      const bool inside = p.group_mode != 1 || t.m0 + quad * 32 + 32 <= t.m_limit;
+      if (MINB == 1 && p.staged && inside) {
         if (has_acc || !p.accumulate) store_tile<BN>(p, t, tmC, epi_stage + quad * (32 * 128), taddr, quad, lane, has_acc);
         if (has_acc) {
           tc_fence_before();

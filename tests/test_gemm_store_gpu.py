@@ -88,3 +88,24 @@ def test_expert_rows(N, K):
         assert ((out[off[e]:off[e + 1]].double() - ref).abs() <= _bound(a, w[e], K) + 2.0 ** -8 * ref.abs()).all()
     assert bool((out[384:] == 5).all())       # rows behind the last segment are not written
     _lib.check_device_errors()
+
+
+@pytest.mark.parametrize("N,K", [(384, 264), (48, 136)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_segments_that_end_inside_a_tile(N, K, dtype):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    rows = [100, 0, 257, 32, 140, 1]
+    off = torch.tensor([0] + rows).cumsum(0).to(torch.int32).cuda()
+    x, w = _rand(g, 640, K), _rand(g, len(rows), N, K)
+    for _ in range(5):
+        out = torch.full((640, N), 5.0, device="cuda", dtype=dtype)
+        G.grouped_gemm(x, w, off, out=out)
+        rnd = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23
+        for e in range(len(rows)):
+            a = x[off[e]:off[e + 1]]
+            ref = a.double() @ w[e].double().t()
+            assert ((out[off[e]:off[e + 1]].double() - ref).abs() <= _bound(a, w[e], K) + rnd * ref.abs()).all()
+        assert bool((out[sum(rows):] == 5).all())
+    _lib.check_device_errors()
