@@ -217,7 +217,8 @@ def _declare_kernels(lib: ctypes.CDLL):
     d("gk_mla_expand", [P, P, P, P, I, I, I, I, I, P])
     d("gk_mla_expand_bwd", [P, P, P, P, I, I, I, I, I, P])
     d("gk_latent_append", [P, L, P, P, P, P, I, I, I, F, F, I, P])
-    d("gk_embedding_grad", [P, P, P, P, I, I, L, P])
+    d("gk_embedding_grad", [P, P, P, P, P, I, I, L, P])
+    d("gk_embedding_grad_scratch", [I, I], L)
     d("gk_decode_begin", [P, P, P])
     d("gk_decode_end", [P, I, I, P])
     d("gk_grpo_loss", [P, P, P, P, P, L, F, F, F, F, F, F, P, P, P, P])

@@ -79,8 +79,8 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6, residual: torch
 
 # ------------------------------------------------------------------------------------------------ embedding
 class _EmbeddingFn(torch.autograd.Function):
-    """Embedding rows; the table's gradient is added to its fp32 ``main_grad`` (rows of equal tokens in the order of the
-    batch), autograd sees none."""
+    """Embedding rows; the table's gradient is added to its fp32 ``main_grad`` (rows of equal tokens in a fixed order),
+    autograd sees none."""
 
     @staticmethod
     def forward(ctx, ids, weight, main_grad):
@@ -95,9 +95,11 @@ class _EmbeddingFn(torch.autograd.Function):
         g = g.reshape(-1, H)
         g = g if g.is_contiguous() and g.data_ptr() % 16 == 0 else g.clone(memory_format=torch.contiguous_format)
         order, rows = torch.sort(ids.reshape(-1), stable=True)
+        lib = _lib.kernels()
+        scratch = torch.empty(lib.gk_embedding_grad_scratch(rows.numel(), H), dtype=torch.float32, device=g.device)
         LAUNCHES["elementwise"] += 1
-        _lib.check(_lib.kernels().gk_embedding_grad(_lib.ptr(order), _lib.ptr(rows), _lib.ptr(g), _lib.ptr(ctx.main_grad),
-                                                    rows.numel(), H, V, _lib.stream_ptr()), "embedding_grad")
+        _lib.check(lib.gk_embedding_grad(_lib.ptr(order), _lib.ptr(rows), _lib.ptr(g), _lib.ptr(ctx.main_grad),
+                                         _lib.ptr(scratch), rows.numel(), H, V, _lib.stream_ptr()), "embedding_grad")
         return None, None, None
 
 

@@ -28,6 +28,31 @@ def test_embedding_gradient(n, V, H):
     assert torch.equal(w.main_grad[V - 1], old[V - 1]) or V == 1
 
 
+@pytest.mark.parametrize("runs", [[128], [129], [1, 127, 1], [5, 250, 1, 128, 128, 3], [256, 256, 1], [1000, 2, 9000], [64, 192, 300]])
+def test_runs_that_cross_blocks(runs):
+    """Runs of equal tokens that end at, before and behind the borders of the kernel's blocks of 128; the same bits each time."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    H, n = 72, sum(runs)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    ids = torch.cat([torch.full((r,), 3 * k, device="cuda") for k, r in enumerate(runs)])
+    ids = ids[torch.randperm(n, generator=g, device="cuda")]
+    w = torch.nn.Parameter(torch.zeros(3 * len(runs), H, device="cuda", dtype=torch.bfloat16))
+    old = torch.randn(w.shape, generator=g, device="cuda")
+    dy = torch.randn(n, H, generator=g, device="cuda").bfloat16()
+    rows = torch.zeros(w.shape, device="cuda", dtype=torch.double).index_add_(0, ids, dy.double())
+    mag = torch.zeros(w.shape, device="cuda", dtype=torch.double).index_add_(0, ids, dy.double().abs())
+    got = []
+    for _ in range(2):
+        w.main_grad = old.clone()
+        fused.embedding(ids, w).backward(dy)
+        # blocks of 128 one after another, then their sums
+        assert ((w.main_grad.double() - old.double() - rows).abs()
+                <= (129 + n // 128) * 2.0 ** -24 * (mag + old.double().abs())).all()
+        got.append(w.main_grad)
+    assert torch.equal(*got)
+
+
 @pytest.mark.parametrize("V,pad", [(40, 0), (1003, 0), (32768, 0), (32768, 3), (4100, 4)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("entropy", [False, True])
