@@ -442,15 +442,16 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict
   }
 }
 
-// The same for aligned rows: 16-byte units, and one angle for all heads of a token, ROPE_TOKENS tokens a CTA.  Rotates the
-// values [off, off + rot) of every head; with y != x the other values are copied.  8000 tokens of 32 heads of 128: 41 us against
-// 84 a pair at a time, 26000 tokens of 40 heads 139 against 309.
-constexpr int ROPE_TOKENS = 4, ROPE_MAX_ROT = 512;
+// The same for aligned rows: 16-byte units, and one angle for all heads of a token.  A CTA takes `tokens` tokens of `heads`
+// heads (grid: tokens, heads).  Rotates the values [off, off + rot) of every head; with y != x the other values are copied.
+// 8000 tokens of 32 heads of 128: 35 us against 68 a pair at a time, 26000 tokens of 40 heads 139 against 309.
+constexpr int ROPE_ANGLES = 1024, ROPE_MAX_ROT = 512;
 __global__ void __launch_bounds__(256) rope_rows_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const int* __restrict__ pos,
                                                         int T, int nheads, int D, int off, int rot, long long ldx, long long ldy,
-                                                        float theta, float sign, int interleaved) {
-  __shared__ float2 cs[ROPE_TOKENS * ROPE_MAX_ROT / 2];
-  const int half = rot >> 1, t0 = blockIdx.x * ROPE_TOKENS, n = T - t0 < ROPE_TOKENS ? T - t0 : ROPE_TOKENS;
+                                                        float theta, float sign, int interleaved, int tokens, int heads) {
+  __shared__ float2 cs[ROPE_ANGLES];   // tokens * rot / 2
+  const int half = rot >> 1, t0 = blockIdx.x * tokens, n = T - t0 < tokens ? T - t0 : tokens;
+  const int h0 = blockIdx.y * heads, nh = nheads - h0 < heads ? nheads - h0 : heads;
   for (int k = threadIdx.x; k < n * half; k += 256) {
     const int tok = k / half, i = k - tok * half;
     const float inv = __powf(theta, -2.f * i / rot);
@@ -461,9 +462,9 @@ __global__ void __launch_bounds__(256) rope_rows_kernel(const __nv_bfloat16* x, 
   __syncthreads();
   const unsigned turned = interleaved ? rot >> 3 : rot >> 4;               // units of a head that rotate: one or two vectors
   const unsigned lead = off >> 3, kept = x == y ? 0 : (D - rot) >> 3;      // vectors that are copied, `lead` of them in front
-  const unsigned per = turned + kept, units = n * nheads * per;
+  const unsigned per = turned + kept, units = n * nh * per;
   for (unsigned u = threadIdx.x; u < units; u += 256) {
-    const unsigned th = u / per, k = u - th * per, tok = th / nheads, h = th - tok * nheads;
+    const unsigned th = u / per, k = u - th * per, tok = th / nh, h = h0 + th - tok * nh;
     const bf16x8* from = reinterpret_cast<const bf16x8*>(x + (t0 + tok) * ldx + static_cast<long long>(h) * D);
     bf16x8* to = reinterpret_cast<bf16x8*>(y + (t0 + tok) * ldy + static_cast<long long>(h) * D);
     if (k >= turned) {
@@ -497,6 +498,31 @@ __global__ void __launch_bounds__(256) rope_rows_kernel(const __nv_bfloat16* x, 
       to[other] = pack8(g);
     }
   }
+}
+
+// A CTA for about 256 units of 16 bytes: several tokens of few heads where there are tokens enough to fill the GPU, a share of
+// the heads where there are not.  128 heads of 128 + 64, the 64 rotated, us, four tokens a CTA -> here (split and rotated in two
+// launches): 1 token 8.6 -> 2.3 (4.5), 32 tokens 28.8 -> 3.0 (6.1), 512 tokens 29.9 -> 14 (21.5), 3400 tokens 93 -> 83 (143).
+static int rope_rows_launch(const void* x, void* y, const int* pos, int T, int nheads, int D, int off, int rot, long long ldx,
+                            long long ldy, float theta, int backward, int interleaved, cudaStream_t st) {
+  const int per = (interleaved ? rot >> 3 : rot >> 4) + (x == y ? 0 : (D - rot) >> 3), sms = sm_count();
+  const long long units = static_cast<long long>(nheads) * per;   // of a token
+  int tokens = 1, gy = 1;
+  if (units < 256) {
+    const int room = 2 * ROPE_ANGLES / rot, spare = T / (2 * sms);
+    tokens = static_cast<int>(256 / units);
+    if (tokens > room) tokens = room;
+    if (tokens > spare) tokens = spare;
+    if (tokens < 1) tokens = 1;
+  } else {
+    gy = (4 * sms + T - 1) / T;
+    if (gy > (units + 255) / 256) gy = static_cast<int>((units + 255) / 256);
+  }
+  const int heads = (nheads + gy - 1) / gy;
+  rope_rows_kernel<<<dim3((T + tokens - 1) / tokens, (nheads + heads - 1) / heads), 256, 0, st>>>(
+      static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), pos, T, nheads, D, off, rot, ldx, ldy, theta,
+      backward ? -1.f : 1.f, interleaved, tokens, heads);
+  return launch_status();
 }
 
 // Same rotation with the angles given as tables cos / sin [T, rot / 2] (multi-axis rotary position ids of
@@ -821,10 +847,8 @@ GK_EXPORT int gk_rope_copy(const void* x, void* y, const int* pos, int T, int nh
   const long long ld = static_cast<long long>(nheads) * D;
   if (x == y || !rope_rows_ok(x, y, D, off, rot, ld, ld, interleaved)) return -1;
   if (T == 0) return 0;
-  rope_rows_kernel<<<(T + ROPE_TOKENS - 1) / ROPE_TOKENS, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), pos, T, nheads, D, off, rot, ld, ld, theta,
-      backward ? -1.f : 1.f, interleaved);
-  return launch_status();
+  return rope_rows_launch(x, y, pos, T, nheads, D, off, rot, ld, ld, theta, backward, interleaved,
+                          reinterpret_cast<cudaStream_t>(stream));
 }
 
 GK_EXPORT int gk_rope(void* x, const int* pos, int T, int nheads, int D, int rot, long long stride_t, float theta,
@@ -832,12 +856,11 @@ GK_EXPORT int gk_rope(void* x, const int* pos, int T, int nheads, int D, int rot
   if (rot % 2 || rot > D) return -1;
   const long long total = static_cast<long long>(T) * nheads * (rot / 2);
   if (total == 0) return 0;
-  if (rope_rows_ok(x, x, D, 0, rot, stride_t, stride_t, interleaved)) {
-    rope_rows_kernel<<<(T + ROPE_TOKENS - 1) / ROPE_TOKENS, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(x), pos, T, nheads, D, 0, rot, stride_t, stride_t,
-        theta, backward ? -1.f : 1.f, interleaved);
-    return launch_status();
-  }
+  // Below about 100k pairs a launch is all latency, and a thread per pair has the shorter chain (us, pairs -> rows: 32 heads of
+  // 128, 16 tokens 1.9 -> 2.4, 64 tokens 2.5 -> 2.5, 512 tokens 6.7 -> 4.4; one head of 64, 1024 tokens 1.9 -> 2.2).
+  if (total >= 98304 && rope_rows_ok(x, x, D, 0, rot, stride_t, stride_t, interleaved))
+    return rope_rows_launch(x, x, pos, T, nheads, D, 0, rot, stride_t, stride_t, theta, backward, interleaved,
+                            reinterpret_cast<cudaStream_t>(stream));
   rope_kernel<<<grid_for(total, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<__nv_bfloat16*>(x), pos, T, nheads, D, rot, stride_t, theta, backward ? -1.f : 1.f,
       interleaved);

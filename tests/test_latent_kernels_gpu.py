@@ -36,6 +36,23 @@ def test_rope_rows(T, heads, D, rot, interleaved):
     assert ((again[:, :heads].double() - back).abs() <= 2.0 ** -8 * back.abs() + _angles_bound(pos, old)).all()
 
 
+# a thread per pair, one below and at the line; several tokens of few heads a CTA, as many as the angles allow; shares of the heads
+@pytest.mark.parametrize("T,heads,D,rot", [(1535, 2, 64, 64), (1536, 2, 64, 64), (9001, 1, 64, 64), (3503, 4, 128, 128),
+                                           (2000, 1, 512, 512), (25, 128, 64, 64), (599, 37, 128, 128)])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_rope_launches(T, heads, D, rot, interleaved):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rows = torch.randn(T, heads + 1, D, generator=g, device="cuda").bfloat16()
+    pos = torch.randint(0, 2000, (T,), generator=g, device="cuda", dtype=torch.int32)
+    old = rows.clone()
+    ref = fused.rope_ref(old[:, :heads].float(), pos, THETA, rot, interleaved).double()
+    fused.rope_inplace(rows[:, :heads], pos, THETA, rot, interleaved)
+    assert ((rows[:, :heads].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + _angles_bound(pos, old)).all()
+    assert torch.equal(rows[:, heads:], old[:, heads:])
+
+
 @pytest.mark.parametrize("T", [1, 6, 301])
 @pytest.mark.parametrize("heads,D,rot", [(1, 32, 16), (5, 192, 64), (128, 192, 64)])
 @pytest.mark.parametrize("interleaved", [False, True])
