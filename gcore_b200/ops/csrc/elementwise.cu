@@ -124,51 +124,6 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
   }
 }
 
-// Rows beyond 8192 values do not fit the registers: two passes over memory.
-__global__ void __launch_bounds__(256) rmsnorm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x,
-                                                               const __nv_bfloat16* __restrict__ res,
-                                                               const __nv_bfloat16* __restrict__ w,
-                                                               __nv_bfloat16* __restrict__ y,
-                                                               __nv_bfloat16* __restrict__ res_out,
-                                                               float* __restrict__ rstd_out, int T, int H, float eps) {
-  __shared__ float red[32];
-  pdl_launch_dependents();
-  pdl_wait();
-  const int nv = H >> 3;
-  auto value = [&](size_t at, float (&f)[8]) {
-    unpack8(reinterpret_cast<const bf16x8*>(x)[at], f);
-    if (res) {
-      float g[8];
-      unpack8(reinterpret_cast<const bf16x8*>(res)[at], g);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] += g[j];
-      unpack8(pack8(f), f);  // what the residual stream stores
-    }
-  };
-  for (int row = blockIdx.x; row < T; row += gridDim.x) {
-    const size_t at = static_cast<size_t>(row) * nv;
-    float ss = 0.f;
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-      float f[8];
-      value(at + i, f);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
-    }
-    ss = block_sum(ss, red);
-    const float rstd = rsqrtf(ss / H + eps);
-    if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-      float f[8], g[8];
-      value(at + i, f);
-      if (res && res_out) reinterpret_cast<bf16x8*>(res_out)[at + i] = pack8(f);
-      unpack8(reinterpret_cast<const bf16x8*>(w)[i], g);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * g[j];
-      reinterpret_cast<bf16x8*>(y)[at + i] = pack8(f);
-    }
-  }
-}
-
 // Rows of at most 256 values (heads): LANES lanes of a warp per row, a CTA of eight warps for 256 / LANES rows.  With a CTA
 // per row 16 of 256 threads had work.
 template <int LANES>
@@ -395,7 +350,7 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const float* __rest
   }
 }
 
-constexpr int RMS_SMALL_H = 256, RMS_MAX_BWD_H = 256 * 8 * 4;
+constexpr int RMS_SMALL_H = 256, RMS_MAX_H = 256 * 8 * 4;
 
 inline int rmsnorm_bwd_launch(const void* g, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
                               float* dw_partial, float* dw, int dw_accumulate, int T, int H, int parts, cudaStream_t st) {
@@ -755,7 +710,7 @@ using namespace gk;
 
 GK_EXPORT int gk_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* res_out, float* rstd,
                              int T, int H, float eps, void* stream) {
-  if (H % 8) return -1;
+  if (H % 8 || H > RMS_MAX_H) return -1;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   auto go = [&](auto kernel, int grid, int threads) {
     launch_k(kernel, dim3(grid > 0 ? grid : 1), dim3(threads), 0, st, static_cast<const __nv_bfloat16*>(x),
@@ -770,8 +725,7 @@ GK_EXPORT int gk_rmsnorm_fwd(const void* x, const void* res, const void* w, void
   const int grid = T < sms * 8 ? T : sms * 8;
   if (nv <= 256) return go(rmsnorm_fwd_kernel<1>, grid, 256);
   if (nv <= 512) return go(rmsnorm_fwd_kernel<2>, grid, 256);
-  if (nv <= 1024) return go(rmsnorm_fwd_kernel<4>, grid, 256);
-  return go(rmsnorm_fwd_wide_kernel, grid, 256);
+  return go(rmsnorm_fwd_kernel<4>, grid, 256);
 }
 
 // Per-head RMSNorm of the query and key heads of packed [q | k | v] rows, in place (decode / prefill of models with
@@ -831,7 +785,7 @@ GK_EXPORT int gk_rmsnorm_bwd_parts(int T) {
 // dw_partial must hold gk_rmsnorm_bwd_parts(T) * H floats.
 GK_EXPORT int gk_rmsnorm_bwd(const void* g, const void* x, const void* w, const float* rstd, const void* dres,
                              void* dx, float* dw_partial, float* dw, int dw_accumulate, int T, int H, void* stream) {
-  if (H % 8 || H > RMS_MAX_BWD_H) return -1;
+  if (H % 8 || H > RMS_MAX_H) return -1;
   return rmsnorm_bwd_launch(g, x, w, rstd, dres, dx, dw_partial, dw, dw_accumulate, T, H, gk_rmsnorm_bwd_parts(T),
                             reinterpret_cast<cudaStream_t>(stream));
 }
