@@ -359,12 +359,15 @@ inline int rmsnorm_bwd_launch(const void* g, const void* x, const void* w, const
   const auto* wp = static_cast<const __nv_bfloat16*>(w);
   const auto* dp = static_cast<const __nv_bfloat16*>(dres);
   auto* op = static_cast<__nv_bfloat16*>(dx);
+  const int rows = H <= 64 ? 32 : H <= 128 ? 16 : H <= RMS_SMALL_H ? 8 : 1;   // of a CTA at a time
+  if (parts > (T + rows - 1) / rows) parts = T > 0 ? (T + rows - 1) / rows : 1;
   auto go = [&](auto kernel) { kernel<<<parts, 256, 0, st>>>(gp, xp, wp, rstd, dp, op, dw_partial, T, H); };
   if (H <= 64) go(rmsnorm_bwd_small_kernel<8>);
   else if (H <= 128) go(rmsnorm_bwd_small_kernel<16>);
   else if (H <= RMS_SMALL_H) go(rmsnorm_bwd_small_kernel<32>);
   else if (H <= 2048) go(rmsnorm_bwd_kernel<1>);
   else if (H <= 4096) go(rmsnorm_bwd_kernel<2>);
+  else if (H <= 6144) go(rmsnorm_bwd_kernel<3>);
   else go(rmsnorm_bwd_kernel<4>);
   colsum_partial_kernel<<<(H + 31) / 32, 256, 0, st>>>(dw_partial, dw, parts, H, dw_accumulate);
   return launch_status();
