@@ -642,8 +642,8 @@ __global__ void __launch_bounds__(256) adam_kernel(const AdamArgs a, long long f
   }
 }
 
-// Every thread keeps four partial sums, over elements `first` and on; VEC (16-byte aligned input): 16 bytes a load, four
-// loads in flight (700 M fp32: 468 us, 6.0 TB/s, against 729 us; 45 M: 47 against 64 us).
+// Every thread keeps four partial sums; VEC (16-byte aligned input): 16 bytes a load, four loads in flight (700 M fp32: 468 us,
+// 6.0 TB/s, against 729 us; 45 M: 47 against 64 us).
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) sumsq_kernel(const T* __restrict__ x, long long n, float* __restrict__ out) {
   __shared__ float red[32];
@@ -891,8 +891,10 @@ GK_EXPORT int gk_adam(float* master, float* m, float* v, const void* grad, int g
 GK_EXPORT int gk_sumsq(const void* x, int is_fp32, long long n, float* out, void* stream) {
   if (n == 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  const int grid = grid_for(n, 256 * (vec ? 16 : 1), 8);
+  const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && n >= 2048;   // below, one element a thread is one load deep
+  // 64 bytes a thread; short inputs one load a thread as far as there are SMs (10000 fp32: 2.6 -> 2.0 us)
+  const int once = grid_for(n * (is_fp32 ? 4 : 2) / 16, 256, 1), four = grid_for(n * (is_fp32 ? 4 : 2) / 64, 256);
+  const int grid = !vec ? grid_for(n, 256, 4) : once > four ? once : four;
   if (is_fp32) {
     const float* f = static_cast<const float*>(x);
     if (vec) sumsq_kernel<float, true><<<grid, 256, 0, st>>>(f, n, out);
