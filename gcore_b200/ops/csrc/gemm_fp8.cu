@@ -252,13 +252,14 @@ static int launch_fp8(const void* A, long long lda, long long a_rows, const void
   return gk::launch_status();
 }
 
-// A wide tile is twice the work at four thirds of the rate: 1.5 narrow ones.  With few K blocks per tile the store counts, which
-// two warps per lane quarter do for twice the columns (3400 x 32768 x 512: 158 us against 147).
+// A wide tile is twice the work.  What it costs, in narrow ones of the same depth (the store is done by two warps per lane
+// quarter for twice the columns, so it weighs more the fewer K blocks there are): 1.86 at K = 768, 1.76 at 1024, 1.61 at 2048,
+// 1.57 at 4096, 1.45 at 7168, or 1.45 + 320 / K.  So two wide waves for three narrow ones lose below a depth of 6000 (3400 x
+// 2048, us, narrow / wide: K = 1024 17.6 / 19.7, 4096 49.5 / 50.7, 7168 85 / 80), one for two win down to 768.
 static bool wide_tiles_pay(int M, int N, int K) {
-  if (K < 1024) return false;
   const long long mt = (M + BM - 1) / BM, sms = gk::sm_count();
   const long long narrow = (mt * ((N + 127) / 128) + sms - 1) / sms, wide = (mt * ((N + 255) / 256) + sms - 1) / sms;
-  return 3 * wide <= 2 * narrow;
+  return wide * (145ll * K + 32000) < narrow * 100 * K;
 }
 
 // A [M,K] and B [N,K] are e4m3 bytes (row-major, K contiguous, K % 16 == 0); sA fp32 [M, ceil(K/128)],
@@ -287,6 +288,8 @@ GK_EXPORT int gk_gemm_fp8_grouped(const void* A, long long lda, const void* B, l
   p.group_offsets = offsets; p.num_groups = num_groups;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const long long b_rows = static_cast<long long>(num_groups) * N;
-  return wide_tiles_pay(M_cap, N, K) ? launch_fp8<256>(A, lda, M_cap, B, ldb, b_rows, p, st)
+  // with one row tile a group every tile brings weights of its own, and the deeper ring of the narrow tiles is what counts
+  // (64 groups of 128 rows, N = 1408, K = 2048: 60 us against 67; of 256 rows: 110 against 107)
+  return M_cap >= 2ll * BM * num_groups && wide_tiles_pay(M_cap, N, K) ? launch_fp8<256>(A, lda, M_cap, B, ldb, b_rows, p, st)
                                   : launch_fp8<128>(A, lda, M_cap, B, ldb, b_rows, p, st);
 }
