@@ -166,7 +166,7 @@ def _declare_kernels(lib: ctypes.CDLL):
     d("gk_gemm_wide_set_staged", [I], None)
     d("gk_gemm_skinny", [P, L, P, L, P, L, I, P, I, I, I, I, I, I, P, P])
     d("gk_gemm_skinny_max_clusters", [I, I, I])
-    d("gk_gemm_stream", [P, L, P, L, P, L, I, P, I, I, I, I, P, L, P, L, P, P])
+    d("gk_gemm_stream", [P, L, P, L, P, L, I, P, I, I, I, I, P, L, P, L, I, P, P])
     d("gk_gemm_stream_scratch", [I], L)
     d("gk_capture_id", [P], ctypes.c_ulonglong)
     d("gk_gemm_comm", [I, P, L, P, L, L, I, P, L, P, I, I, I, I, I, I, I, ctypes.c_uint, P, L, P, P])

@@ -41,6 +41,7 @@ struct StParams {
   int bias_fp32;
   float* ws;       // [CTA][first, last piece][Tp tokens][128 features]
   unsigned long long* counters;   // [tiles]: pieces there | CTAs done << 8 | shares left over << 16, zero between launches
+  int share_wait;  // cycles a CTA waits for the others' pieces before it leaves its share of the tile to the last one
   int* err;
 };
 
@@ -89,7 +90,6 @@ __device__ __forceinline__ unsigned long long load_acquire(const unsigned long l
   return v;
 }
 constexpr int MAX_PIECES = 48;             // shares of a tile the counter word has a bit for
-constexpr long long SHARE_WAIT = 100000;   // cycles, about 50 us
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
 // Adds up items [i0, i1) of a divided tile, an item being four features of one token.
@@ -159,7 +159,7 @@ __device__ __forceinline__ void finish_piece(const StParams& p, int tile, int ct
       } else {
         const long long t0 = clock64();
         while (static_cast<int>(load_acquire(word) & 0xff) < pieces) {
-          if (clock64() - t0 < SHARE_WAIT) continue;
+          if (clock64() - t0 < p.share_wait) continue;
           // the CTA that brings the last piece sees the bit, unless it came first: then all pieces are there
           if (static_cast<int>(atomicOr(word, shares << 16) & 0xff) < pieces) shares = 0;
           break;
@@ -344,10 +344,11 @@ GK_EXPORT long long gk_gemm_stream_scratch(int T) { return 2ll * sm_count() * pa
 
 // W [N, K] and X [T, K] bf16 row-major (K contiguous, leading dimensions multiples of 8, 16-byte aligned), 1 <= T <= 128.
 // counters: two zero ints per 128 features, 8-byte aligned; a launch leaves them at zero, and launches that may run at the
-// same time must not share them.
+// same time must not share them.  share_wait: cycles a CTA waits for the other pieces of its tile (results do not depend on it).
 GK_EXPORT int gk_gemm_stream(const void* W, long long ldw, const void* X, long long ldx, void* Y, long long ldy,
                              int out_fp32, const void* bias, int bias_fp32, int T, int N, int K, float* ws,
-                             long long ws_floats, int* counters, long long counter_ints, int* err, void* stream) {
+                             long long ws_floats, int* counters, long long counter_ints, int share_wait, int* err,
+                             void* stream) {
   if (T < 1 || T > 128 || N < 1 || K < 1) return -1;
   if ((ldw & 7) || (ldx & 7) || (reinterpret_cast<uintptr_t>(W) & 15) || (reinterpret_cast<uintptr_t>(X) & 15)) return -3;
   StParams p;
@@ -362,7 +363,8 @@ GK_EXPORT int gk_gemm_stream(const void* W, long long ldw, const void* X, long l
   if (make_tmap_2d(&tmW, W, 2, N, K, ldw, BM, BK, true)) return -4;
   if (make_tmap_2d(&tmX, X, 2, T, K, ldx, p.Tp, BK, true)) return -5;
   p.Y = Y; p.ldy = ldy; p.out_fp32 = out_fp32; p.bias = bias; p.bias_fp32 = bias_fp32;
-  p.ws = ws; p.counters = reinterpret_cast<unsigned long long*>(counters); p.err = err;
+  p.ws = ws; p.counters = reinterpret_cast<unsigned long long*>(counters);
+  p.share_wait = share_wait; p.err = err;
   const int sms = sm_count(), stage_bytes = A_BYTES + p.Tp * 128;
   const double weight_us = 2e-6 * N * K / 6.5;   // time the weight takes from HBM
   // Ring: below half of an SM the next GEMM's CTA fits beside this one and has its first loads under way early; that pays

@@ -275,6 +275,7 @@ def _skinny_plan(T: int, tiles: int, kb: int, K: int):
 STREAM = {"enabled": os.environ.get("GCORE_STREAM_GEMM", "1") != "0"}
 _STREAM_SCRATCH: dict = {}  # tokens -> floats of scratch
 COUNTER_INTS, COUNTER_OWNERS = 8192, 64
+SHARE_WAIT = 100000    # cycles, about 50 us: a CTA whose tile is not complete by then leaves its share to the last one
 _COUNTERS: dict = {}   # (device, stream) -> counters of divided tiles, zero between launches
 _CAPTURED: dict = {}   # (device, stream, capture) -> the same in a capture under way
 
@@ -341,7 +342,8 @@ def linear_forward(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None =
             rc = lib.gk_gemm_stream(
                 w.data_ptr(), w.stride(0), x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0),
                 y.dtype == torch.float32, _lib.ptr(bias), bias is not None and bias.dtype == torch.float32, T, N, K,
-                ws.data_ptr(), floats, counters.data_ptr(), counters.numel(), _lib.err_flag(x.device).data_ptr(), stream)
+                ws.data_ptr(), floats, counters.data_ptr(), counters.numel(), SHARE_WAIT, _lib.err_flag(x.device).data_ptr(),
+                stream)
             _lib.check(rc, "gk_gemm_stream")
             return y
         bn = 32 if T <= 32 else (64 if T <= 64 else 128)

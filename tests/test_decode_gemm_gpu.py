@@ -184,3 +184,22 @@ def test_ends_while_an_earlier_error_stands(N, K):
             _lib.check_device_errors()
         assert torch.equal(G.linear_forward(x, w, out_dtype=torch.float32), ref)
     _lib.check_device_errors()
+
+
+# few feature tiles: one piece per CTA; 4 to 48 pieces a tile, ragged ones among them
+@pytest.mark.parametrize("N,K", [(4608, 1600), (2048, 4096), (700, 9000), (300, 20000)])
+@pytest.mark.parametrize("T", [1, 17, 128])
+def test_shares_left_to_the_last_piece(N, K, T, monkeypatch):
+    """Without patience every CTA but the one that brings a tile's last piece leaves its share to that one."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    g = torch.Generator(device="cuda").manual_seed(N + K + T)
+    x = torch.randn(T, K, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    ref = G.linear_forward(x, w, out_dtype=torch.float32)
+    monkeypatch.setattr(G, "SHARE_WAIT", 0)
+    for _ in range(20):                                      # on the same counters, which have to be back at zero
+        assert torch.equal(G.linear_forward(x, w, out_dtype=torch.float32), ref)
+    torch.cuda.synchronize()
+    assert all(not c.any() for c in G._COUNTERS.values())
+    _lib.check_device_errors()
