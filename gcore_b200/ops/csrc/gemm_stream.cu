@@ -386,11 +386,15 @@ GK_EXPORT int gk_gemm_stream(const void* W, long long ldw, const void* X, long l
     if (ks > MAX_PIECES) ks = MAX_PIECES;
     if (full || ks == most || ks == MAX_PIECES || T > 64) { p.ks = ks; grid = tiles * ks; }
   }
-  // Adding up divided tiles costs about 1.5 us and 0.1 us per token; whole tiles leave SMs idle in the last round
-  // (32768 x 1024, 64 tokens: 22.6 in runs, 18.2 in whole tiles; 28672 x 4096, 4 tokens: 42 against 52).
-  if (!p.ks && tiles >= sms) {
+  // Adding up divided tiles costs about 1.5 us and 0.1 us per token, with fewer tiles than SMs (where hardly one is whole) 4 us
+  // and 0.14; whole tiles leave SMs idle in the last round (runs / whole, us: 32768 x 1024, 64 tokens 22.6 / 18.2; 28672 x 4096,
+  // 4 tokens 42 / 52; 10240 x 1024, 4 and 64 tokens 12.5 / 10.7 and 22 / 11.9; 9728 x 5120 24 / 34 and 33 / 36).
+  if (!p.ks && 2 * tiles > sms) {
     const double rounds = (tiles + sms - 1) / sms, idle_us = (rounds * sms / tiles - 1.) * weight_us;
-    if (idle_us < 1.5 + 0.1 * T) p.tiles = tiles;
+    if (idle_us < (tiles < sms ? 4. + 0.14 * T : 1.5 + 0.1 * T)) {
+      p.tiles = tiles;
+      grid = tiles < sms ? tiles : sms;
+    }
   }
   static bool configured = false;
   if (!configured) {

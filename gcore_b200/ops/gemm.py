@@ -272,6 +272,17 @@ def _skinny_plan(T: int, tiles: int, kb: int, K: int):
     return plan
 
 
+def _cluster_quicker(T: int, tiles: int, kb: int, K: int) -> bool:
+    """Whether the cluster kernel beats the weight-streaming one on a weight of its range (few tiles, moderate K): few
+    tokens, whose sums cost it little in distributed shared memory, and a cluster of eight or four CTAs per tile (us, cluster
+    / stream: 1024 x 5120, 4 and 32 tokens 9.2 / 11.4 and 10.2 / 11.7; 1536 x 7168 11.4 / 12.5 and 12.2 / 12.5; 4096 x 4096,
+    4 tokens 13.3 / 14.1; odd cluster sizes: 2048 x 4096 12.6 / 11.4)."""
+    if not _SKINNY[0] or T > 48 or tiles > SKINNY_MAX_TILES[0] or kb > 160:
+        return False
+    ks = _skinny_plan(T, tiles, kb, K)[0]
+    return (ks == 8 and (T <= 32 or kb <= 112)) or (ks == 4 and T <= 16)
+
+
 STREAM = {"enabled": os.environ.get("GCORE_STREAM_GEMM", "1") != "0"}
 _STREAM_SCRATCH: dict = {}  # tokens -> floats of scratch
 COUNTER_INTS, COUNTER_OWNERS = 8192, 64
@@ -327,7 +338,9 @@ def linear_forward(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None =
     if _lib.use_native(x) and T <= 128 and N >= 256:
         # small weights: the cluster kernel's reduction through distributed shared memory is quicker than the scratch (us, 4
         # tokens: 1024 x 2816 5.6 against 6.7, 576 x 7168 8.2 against 8.5; 5632 x 1024 8.3 against 6.7)
-        if (STREAM["enabled"] and T >= 1 and N * K >= 5 << 20 and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+        tiles, kb = (N + 127) // 128, (K + 63) // 64
+        if (STREAM["enabled"] and T >= 1 and N * K >= 5 << 20 and not _cluster_quicker(T, tiles, kb, K)
+                and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
                 and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
                 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
                 and (out is None or (out.dtype in (torch.bfloat16, torch.float32) and out.stride(1) == 1))
@@ -347,8 +360,6 @@ def linear_forward(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None =
             _lib.check(rc, "gk_gemm_stream")
             return y
         bn = 32 if T <= 32 else (64 if T <= 64 else 128)
-        tiles = (N + 127) // 128
-        kb = (K + 63) // 64
         # measured on B200 under graph replay: the cluster kernel wins for few tiles and moderate K (projections of a
         # tensor-parallel shard); the persistent kernel's global split-K wins for more tiles or very long K
         if (tiles <= SKINNY_MAX_TILES[0] and kb <= 160 and _SKINNY[0] and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16

@@ -9,8 +9,9 @@ pytestmark = pytest.mark.gpu
 
 
 # (N, K): one piece per CTA with equal and unequal pieces, ragged tiles and k-blocks, runs that divide tiles, runs of whole
-# tiles, one tile more than SMs
-SHAPES = [(3584, 3584), (4608, 1600), (700, 9000), (7168, 1152), (24576, 512), (32768, 520), (19072, 712), (300, 20000)]
+# tiles, one tile more than SMs; more than half as many tiles as SMs, whole and divided
+SHAPES = [(3584, 3584), (4608, 1600), (700, 9000), (7168, 1152), (24576, 512), (32768, 520), (19072, 712), (300, 20000),
+          (9600, 1024), (9728, 2560), (13000, 416)]
 
 
 @pytest.mark.parametrize("N,K", SHAPES)
@@ -43,7 +44,7 @@ def test_streams_and_captured_branches_keep_their_counters_apart():
     """Launches that may overlap: four streams at once, and two branches of one graph."""
     if not torch.cuda.is_available():
         pytest.skip("needs a GPU")
-    T, N, K = 8, 3584, 4096
+    T, N, K = 8, 4608, 4096
     g = torch.Generator(device="cuda").manual_seed(3)
     xs = [torch.randn(T, K, generator=g, device="cuda").bfloat16() for _ in range(4)]
     w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
@@ -83,7 +84,7 @@ def test_refuses_a_weight_of_another_width(N, K):
 
 
 def _problem(seed, n=2):
-    T, N, K = 8, 3584, 4096
+    T, N, K = 8, 4608, 4096
     g = torch.Generator(device="cuda").manual_seed(seed)
     xs = [torch.randn(T, K, generator=g, device="cuda").bfloat16() for _ in range(n)]
     w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
@@ -168,7 +169,7 @@ def test_counters_start_over_after_a_reported_error():
     _lib.check_device_errors()
 
 
-@pytest.mark.parametrize("N,K", [(3584, 3584), (24576, 512), (32768, 520)])
+@pytest.mark.parametrize("N,K", [(4608, 3584), (24576, 512), (32768, 520)])
 def test_ends_while_an_earlier_error_stands(N, K):
     """Another kernel's error makes waits give up early: the launch ends, and the one after the report is right."""
     if not torch.cuda.is_available():
