@@ -603,14 +603,19 @@ int launch_gemm_q(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensor
 }
 
 template <int BN, bool A_MN, bool B_MN>
-int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int grid, cudaStream_t st) {
+int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, long long tiles, int grid,
+                cudaStream_t st) {
   using C = Cfg<BN>;
   GemmParams q = p;
   // C's planes as a tensor map: one per group of a ragged contraction, else one.  64 bf16 columns a copy need a tile of
   // whole pairs of 32.  Copies are clipped at 16 bytes, so rows have to be whole multiples of that.
+  // A bf16 result of few tiles, or of one k-block, is left to the threads: they wait for no copy at the end, and its bytes are not
+  // what counts (us, threads / TMA: 8 tiles 9.3 / 10.0, 20 tiles 17.4 / 18.0, 40 tiles 12.3 / 12.5, 110 tiles 14.3 / 13.0;
+  // 4096 x 2048 of depth 64 10.4 / 11.5, 4096 x 4096 of depth 256 22.5 / 17.0; fp32, 16 tiles: 10.3 / 9.7).
   const int esz = p.out_fp32 ? 4 : 2;
+  const bool many = p.out_fp32 || (2 * tiles > sm_count() && p.K > BK);
   const long long plane = p.group_mode == 2 ? p.c_group_stride : p.ldc * p.M;
-  q.staged = !p.transposed && p.ksplit == 1 && (p.out_fp32 || (!p.accumulate && BN % 64 == 0)) &&
+  q.staged = many && !p.transposed && p.ksplit == 1 && (p.out_fp32 || (!p.accumulate && BN % 64 == 0)) &&
              (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 && (p.ldc * esz) % 16 == 0 && (plane * esz) % 16 == 0 &&
              (static_cast<long long>(p.N) * esz) % 16 == 0 &&
              plane * esz < (1ll << 40);
@@ -713,11 +718,11 @@ GK_EXPORT int gk_gemm_bf16(const void* A, long long lda, long long a_rows, int a
 
 #define GK_DISPATCH(BN_)                                                                   \
   if (bn == BN_) {                                                                         \
-    if (!a_mn && !b_mn) return launch_gemm<BN_, false, false>(tmA, tmB, p, grid, st);      \
-    if (a_mn && !b_mn) return launch_gemm<BN_, true, false>(tmA, tmB, p, grid, st);        \
+    if (!a_mn && !b_mn) return launch_gemm<BN_, false, false>(tmA, tmB, p, tiles, grid, st); \
+    if (a_mn && !b_mn) return launch_gemm<BN_, true, false>(tmA, tmB, p, tiles, grid, st); \
     if constexpr (BN_ >= 64) {                                                             \
-      if (!a_mn && b_mn) return launch_gemm<BN_, false, true>(tmA, tmB, p, grid, st);      \
-      if (a_mn && b_mn) return launch_gemm<BN_, true, true>(tmA, tmB, p, grid, st);        \
+      if (!a_mn && b_mn) return launch_gemm<BN_, false, true>(tmA, tmB, p, tiles, grid, st); \
+      if (a_mn && b_mn) return launch_gemm<BN_, true, true>(tmA, tmB, p, tiles, grid, st); \
     }                                                                                      \
   }
   GK_DISPATCH(32)
@@ -726,8 +731,8 @@ GK_EXPORT int gk_gemm_bf16(const void* A, long long lda, long long a_rows, int a
   GK_DISPATCH(192)
   GK_DISPATCH(256)
   if (bn == 224 && !b_mn) {  // 224 is not a whole number of 64-column chunks, which the MN-major B loads need
-    if (!a_mn) return launch_gemm<224, false, false>(tmA, tmB, p, grid, st);
-    return launch_gemm<224, true, false>(tmA, tmB, p, grid, st);
+    if (!a_mn) return launch_gemm<224, false, false>(tmA, tmB, p, tiles, grid, st);
+    return launch_gemm<224, true, false>(tmA, tmB, p, tiles, grid, st);
   }
 #undef GK_DISPATCH
   return -16;

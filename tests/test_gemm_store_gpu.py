@@ -18,9 +18,10 @@ def _bound(a, b, K):
     return 4 * K ** 0.5 * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t()) + 1e-12
 
 
-# (M, N, K): 256 x 256 tiles with ragged rows and columns, a partial last wave, 128-row tiles, one narrow tile
+# (M, N, K): 256 x 256 tiles with ragged rows and columns, a partial last wave, 128-row tiles, one narrow tile; more than half as
+# many 128-row tiles as SMs, of several k-blocks and of one
 @pytest.mark.parametrize("M,N,K", [(1100, 2052, 520), (2049, 4100, 264), (300, 200, 136), (129, 264, 72), (40, 36, 64),
-                                   (1100, 2050, 520), (300, 201, 136)])
+                                   (1100, 2050, 520), (300, 201, 136), (900, 2600, 136), (900, 2600, 64)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_dense(M, N, K, dtype):
     if not torch.cuda.is_available():
@@ -72,7 +73,7 @@ def test_weight_gradient_of_experts(N, K):
     _lib.check_device_errors()
 
 
-@pytest.mark.parametrize("N,K", [(384, 264), (200, 72), (48, 136)])
+@pytest.mark.parametrize("N,K", [(384, 264), (200, 72), (48, 136), (4096, 136)])
 def test_expert_rows(N, K):
     if not torch.cuda.is_available():
         pytest.skip("needs a GPU")
@@ -90,7 +91,7 @@ def test_expert_rows(N, K):
     _lib.check_device_errors()
 
 
-@pytest.mark.parametrize("N,K", [(384, 264), (48, 136)])
+@pytest.mark.parametrize("N,K", [(384, 264), (48, 136), (4096, 136)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_segments_that_end_inside_a_tile(N, K, dtype):
     if not torch.cuda.is_available():
