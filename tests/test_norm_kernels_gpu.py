@@ -8,7 +8,7 @@ from gcore_b200.ops import fused
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("H", [8, 64, 72, 128, 136, 256, 264, 1024, 1032, 2048, 2056, 4096, 4104, 7168, 8192])
+@pytest.mark.parametrize("H", [8, 64, 72, 128, 136, 256, 264, 1024, 1032, 2048, 2056, 4096, 4104, 6144, 6152, 7168, 8192])
 @pytest.mark.parametrize("T", [1, 17, 297, 2401])
 @pytest.mark.parametrize("residual", [False, True])
 def test_rmsnorm(H, T, residual):
