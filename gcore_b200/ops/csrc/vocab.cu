@@ -177,10 +177,10 @@ __global__ void __launch_bounds__(256) logprob_entropy_bwd_kernel(T* __restrict_
 // into blocks of EMB_BLOCK.  The CTA at the first of a run of equal tokens, and the one at every block that begins inside a run,
 // adds up the run's rows in its block, in order.  A run inside one block goes straight into the table; the parts of a longer
 // one lie in `part` (two rows a block: what continues from the block before, and what goes on behind it) and
-// embedding_runs_kernel adds them up in order.  Always the same order of additions.  26000 x 4096 with 0, 1000 and
-// 20000 equal ids, forward and backward, us: 339, 366, 370; with one CTA column walking a whole run 331, 833, 11400; autograd's
-// operation 2430, 2410, 1860.  There the sum was a dense bf16 table, cleared, converted and added to the fp32 one.  With the logits' gradient above, policy updates: dense
-// 31.2 -> 30.2 ms, mixture of experts 11.9 -> 11.1.
+// embedding_runs_kernel adds them up in order.  Always the same order of additions.  26000 x 4096 with 0, 1000 and 20000 equal
+// ids, forward and backward, us: 339, 366, 370; with one CTA walking a whole run 331, 833, 11400; autograd's operation 2430,
+// 2410, 1860 (there the sum was a dense bf16 table, cleared, converted and added to the fp32 one).  With the logits' gradient
+// above, policy updates: dense 31.2 -> 30.2 ms, mixture of experts 11.9 -> 11.1.
 constexpr int EMB_BLOCK = 128;
 __device__ __forceinline__ void add8(const uint4& v, float (&acc)[8]) {
   const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
