@@ -801,9 +801,9 @@ static bool rope_rows_ok(const void* x, const void* y, int D, int off, int rot, 
 // y = x [T, nheads, D] (contiguous rows, 16-byte aligned, y != x) with the values [off, off + rot) of every head rotated.
 GK_EXPORT int gk_rope_copy(const void* x, void* y, const int* pos, int T, int nheads, int D, int off, int rot, float theta,
                            int backward, int interleaved, void* stream) {
+  if (T == 0 || nheads == 0) return 0;   // both null then
   const long long ld = static_cast<long long>(nheads) * D;
   if (x == y || !rope_rows_ok(x, y, D, off, rot, ld, ld, interleaved)) return -1;
-  if (T == 0) return 0;
   return rope_rows_launch(x, y, pos, T, nheads, D, off, rot, ld, ld, theta, backward, interleaved,
                           reinterpret_cast<cudaStream_t>(stream));
 }

@@ -7,7 +7,7 @@ from gcore_b200.ops import fused, vocab
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,V,H", [(1, 10, 8), (13, 4, 264), (900, 50, 2048), (5000, 3000, 2056)])
+@pytest.mark.parametrize("n,V,H", [(0, 5, 16), (1, 10, 8), (13, 4, 264), (900, 50, 2048), (5000, 3000, 2056)])
 def test_embedding_gradient(n, V, H):
     if not torch.cuda.is_available():
         pytest.skip("needs a GPU")

@@ -53,8 +53,8 @@ def test_rope_launches(T, heads, D, rot, interleaved):
     assert torch.equal(rows[:, heads:], old[:, heads:])
 
 
-@pytest.mark.parametrize("T", [1, 6, 301])
-@pytest.mark.parametrize("heads,D,rot", [(1, 32, 16), (5, 192, 64), (128, 192, 64)])
+@pytest.mark.parametrize("T", [0, 1, 6, 301])
+@pytest.mark.parametrize("heads,D,rot", [(0, 192, 64), (1, 32, 16), (5, 192, 64), (128, 192, 64)])
 @pytest.mark.parametrize("interleaved", [False, True])
 def test_rotated_tail(T, heads, D, rot, interleaved):
     if not torch.cuda.is_available():
@@ -71,7 +71,7 @@ def test_rotated_tail(T, heads, D, rot, interleaved):
         assert torch.equal(have[..., :D - rot], src[..., :D - rot]) and torch.equal(have[..., D - rot:], tail)
 
 
-@pytest.mark.parametrize("T,h,dn,dr,dv", [(1, 1, 8, 8, 8), (5, 3, 128, 64, 128), (301, 128, 128, 64, 128), (7, 9, 64, 256, 40)])
+@pytest.mark.parametrize("T,h,dn,dr,dv", [(0, 3, 128, 64, 128), (1, 1, 8, 8, 8), (5, 3, 128, 64, 128), (301, 128, 128, 64, 128), (7, 9, 64, 256, 40)])
 def test_expanded_latent(T, h, dn, dr, dv):
     if not torch.cuda.is_available():
         pytest.skip("needs a GPU")
