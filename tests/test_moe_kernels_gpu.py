@@ -125,3 +125,22 @@ def test_decode_layer(T, H, F, E, K, kind, skew):
     err, other = ((z.double() - ref).norm() / ref.norm() for z in (y, general))
     assert err <= 1.05 * other + 1e-4
     _lib.check_device_errors()
+
+
+def test_decode_layer_ends_while_an_earlier_error_stands():
+    """Another kernel's error makes waits give up early: the launches end, and the ones after the report are right."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    g = torch.Generator(device="cuda").manual_seed(1)
+    layer = _layer(1024, 256, 64, 8, "softmax", g)
+    x = torch.randn(40, 1024, generator=g, device="cuda").bfloat16()
+    with torch.no_grad():
+        assert layer._decode_ready(x)
+        ref, _ = layer(x)
+        for _ in range(5):
+            _lib.err_flag(x.device).fill_(1)
+            layer(x)
+            with pytest.raises(RuntimeError, match="timed-out wait"):
+                _lib.check_device_errors()
+            assert torch.equal(layer(x)[0], ref)
+    _lib.check_device_errors()
